@@ -9,6 +9,8 @@
 
 #include <cuda_runtime.h>
 
+#include "fk_fixed.cuh"
+
 namespace fk {
 
 constexpr double kGobet = -0.5826;  // Gobet-Menozzi shift, FeynmanKacSolver.cpp:169,184
@@ -50,15 +52,11 @@ __device__ __forceinline__ uint4 philox10_rk(uint4 c, const uint32_t* rk) {
 }
 
 // Box-Muller pair from two 32-bit words: u = (word + 1/2) 2^-32 in (0,1).
+// FP64 stepping forms it on the integer pipes (fx::normal_pair, about 230
+// issue slots): the FP64 log, square root and sincos were about 70 of a
+// step's 225 FP64 instructions, 64 slots each.
 __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, double& z0, double& z1) {
-  const double inv32 = 2.3283064365386962890625e-10;
-  const double u1 = (static_cast<double>(a) + 0.5) * inv32;
-  const double u2 = (static_cast<double>(b) + 0.5) * inv32;
-  const double rad = sqrt(-2.0 * log(u1));
-  double s, c;
-  sincos(6.283185307179586 * u2, &s, &c);
-  z0 = rad * c;
-  z1 = rad * s;
+  fx::normal_pair(a, b, z0, z1);
 }
 // FP32 stepping uses the SFU forms (ex2/lg2.approx, sqrt.approx and an
 // approximate division): relative errors ~1e-6 at most, far below the Monte
@@ -71,7 +69,12 @@ __device__ __forceinline__ float fexp2(float v) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-__device__ __forceinline__ double fexp(double v) { return exp(v); }
+// e^v: integer pipes for |v| < 256 (fx::exp_core), which holds every exponent of the
+// registered problems near their domains and every stencil weight that is added
+static __device__ __noinline__ double fexp_far(double v) { return exp(v); }
+__device__ __forceinline__ double fexp(double v) {
+  return (static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu) < 0x40700000u ? fx::exp_core(v) : fexp_far(v);
+}
 __device__ __forceinline__ float fsqrt(float v) {
   float r;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -283,6 +286,56 @@ struct FrankeEval {
   }
 };
 
+// FP64 stepping: the Franke function in fixed point where fx::to_pos holds
+// (the unit square and its surroundings), the FP64 forms elsewhere.
+static __device__ __noinline__ void franke_far(double x, double y, bool grad, double& u, double& lap, double& ux, double& uy) {
+  const FrankeEval<double> F(x, y);
+  u = F.u();
+  lap = F.lap();
+  if (grad) {
+    ux = F.ux();
+    uy = F.uy();
+  }
+}
+// Laplacian, and the gradient if asked for.
+__device__ __forceinline__ void franke_lap_grad(double x, double y, bool grad, double& lap, double& ux, double& uy) {
+  fx::i64 X, Y;
+  const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
+  if (!ok) {
+    double u;
+    franke_far(x, y, grad, u, lap, ux, uy);
+    return;
+  }
+  fx::FrankeArgs f;
+  fx::franke_args(X, Y, f);
+  if (grad) {
+    fx::FrankeTerms b;
+    fx::i64 gx, gy;
+    fx::franke_terms(f, b);
+    fx::franke_grad(f, b, gx, gy);
+    ux = fx::to_double(gx, -58);
+    uy = fx::to_double(gy, -58);
+    lap = fx::to_double(fx::franke_lap_terms(f, b), -54);
+  } else {
+    lap = fx::to_double(fx::franke_lap(f), -54);
+  }
+}
+__device__ __forceinline__ double franke_value(double x, double y) {
+  fx::i64 X, Y;
+  const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
+  if (!ok) {
+    double u, lap, ux, uy;
+    franke_far(x, y, false, u, lap, ux, uy);
+    return u;
+  }
+  fx::FrankeArgs f;
+  fx::FrankeTerms b;
+  fx::franke_args(X, Y, f);
+  fx::franke_terms(f, b);
+  return fx::to_double(fx::franke_u(b), -60);
+}
+__device__ __forceinline__ float franke_value(float x, float y) { return FrankeEval<float>(x, y).u(); }
+
 // sin(pi v): SFU form for FP32 stepping (|v| <= 2 here), accurate for FP64
 __device__ __forceinline__ float sinpi_(float v) { return __sinf(3.14159265358979323846f * v); }
 __device__ __forceinline__ double sinpi_(double v) { return sinpi(v); }
@@ -333,19 +386,29 @@ struct Problem<0> {
   __device__ static R sigma_of(R) { return R(1.41421356237); }
   template <typename R>
   __device__ static void step(const BvpDev&, R x, R y, R, R, bool cv, StepCoef<R>& o) {
-    FrankeEval<R> F(x, y);
     o.s = R(1.41421356237);
-    o.f = -F.lap();
     o.c = R(0);
     o.bx = R(0);
     o.by = R(0);
-    if (cv) {
-      o.Fx = -o.s * F.ux();
-      o.Fy = -o.s * F.uy();
+    if constexpr (std::is_same<R, double>::value) {
+      double lap, ux, uy;
+      franke_lap_grad(x, y, cv, lap, ux, uy);
+      o.f = -lap;
+      if (cv) {
+        o.Fx = -o.s * ux;
+        o.Fy = -o.s * uy;
+      }
+    } else {
+      FrankeEval<R> F(x, y);
+      o.f = -F.lap();
+      if (cv) {
+        o.Fx = -o.s * F.ux();
+        o.Fy = -o.s * F.uy();
+      }
     }
   }
   template <typename R>
-  __device__ static R u(const BvpDev&, R x, R y) { return FrankeEval<R>(x, y).u(); }
+  __device__ static R u(const BvpDev&, R x, R y) { return franke_value(x, y); }
 };
 
 // FK_PROBLEM_MONEGROS: sigma = 1.41421356237 I, b = 0, c = -1, f = -Lap u + u.
@@ -380,11 +443,24 @@ struct Problem<2> {
     return R(1) + R(0.5) * sinpi_(R(2) * x) * sinpi_(R(2) * y);
   }
   template <typename R>
-  __device__ static R state(const BvpDev&, R x, R y) { return coef_a(x, y); }
+  __device__ static R state(const BvpDev&, R x, R y) {
+    if constexpr (std::is_same<R, double>::value) {
+      fx::i64 X, Y;
+      if (fx::to_pos(x, X) & fx::to_pos(y, Y)) return fx::to_double(fx::aniso_a(X, Y), 0u, -62);
+      return a_far(x, y);
+    } else {
+      return coef_a(x, y);
+    }
+  }
+  __device__ __noinline__ static double a_far(double x, double y) { return coef_a(x, y); }
   template <typename R>
-  __device__ static R sigma_of(R a) { return fsqrt(R(2) * a); }
+  __device__ static R sigma_of(R a) {
+    // (a is 1/2 to 3/2: sqrt(2a) on the integer pipes)
+    if constexpr (std::is_same<R, double>::value) return fx::aniso_sigma(fx::a_bits(a));
+    else return fsqrt(R(2) * a);
+  }
   template <typename R>
-  __device__ static void step(const BvpDev&, R x, R y, R a, R s, bool cv, StepCoef<R>& o) {
+  __device__ __forceinline__ static void step_of(R x, R y, R a, R s, bool cv, StepCoef<R>& o) {
     FrankeEval<R> F(x, y);
     const R q = R(1) + x * y;
     const R Fv = F.u(), Fx = F.ux(), Fy = F.uy();
@@ -401,8 +477,36 @@ struct Problem<2> {
       o.Fy = -o.s * uy;
     }
   }
+  __device__ __noinline__ static void step_far(double x, double y, double a, double s, bool cv, StepCoef<double>& o) {
+    step_of<double>(x, y, a, s, cv, o);
+  }
   template <typename R>
-  __device__ static R u(const BvpDev&, R x, R y) { return FrankeEval<R>(x, y).u() * (R(1) + x * y); }
+  __device__ static void step(const BvpDev&, R x, R y, R a, R s, bool cv, StepCoef<R>& o) {
+    if constexpr (std::is_same<R, double>::value) {
+      fx::i64 X, Y;
+      if (!(fx::to_pos(x, X) & fx::to_pos(y, Y))) {
+        step_far(x, y, a, s, cv, o);
+        return;
+      }
+      fx::AnisoOut p;
+      fx::aniso_step(X, Y, fx::a_bits(a), p);
+      o.s = s;
+      o.c = -fx::to_double(p.mc, 0u, -54);
+      o.bx = y - 0.5;
+      o.by = 0.5 - x;
+      o.f = fx::to_double(p.f, -51);
+      if (cv) {
+        fx::i64 ux, uy;
+        fx::aniso_grad(X, Y, p, ux, uy);
+        o.Fx = -s * fx::to_double(ux, -54);
+        o.Fy = -s * fx::to_double(uy, -54);
+      }
+    } else {
+      step_of<R>(x, y, a, s, cv, o);
+    }
+  }
+  template <typename R>
+  __device__ static R u(const BvpDev&, R x, R y) { return franke_value(x, y) * (R(1) + x * y); }
 };
 
 // FK_PROBLEM_DISK: Franke mapped from the disk's bounding box to [0,1]^2.
@@ -416,21 +520,31 @@ struct Problem<3> {
   __device__ static void step(const BvpDev& b, R x, R y, R, R, bool cv, StepCoef<R>& o) {
     const R inv = R(1) / (R(2) * R(b.prob[2]));
     const R xi = (x - R(b.prob[0])) * inv + R(0.5), eta = (y - R(b.prob[1])) * inv + R(0.5);
-    FrankeEval<R> F(xi, eta);
     o.s = R(1.41421356237);
-    o.f = -F.lap() * (inv * inv);
     o.c = R(0);
     o.bx = R(0);
     o.by = R(0);
-    if (cv) {
-      o.Fx = -o.s * F.ux() * inv;
-      o.Fy = -o.s * F.uy() * inv;
+    if constexpr (std::is_same<R, double>::value) {
+      double lap, ux, uy;
+      franke_lap_grad(xi, eta, cv, lap, ux, uy);
+      o.f = -lap * (inv * inv);
+      if (cv) {
+        o.Fx = -o.s * ux * inv;
+        o.Fy = -o.s * uy * inv;
+      }
+    } else {
+      FrankeEval<R> F(xi, eta);
+      o.f = -F.lap() * (inv * inv);
+      if (cv) {
+        o.Fx = -o.s * F.ux() * inv;
+        o.Fy = -o.s * F.uy() * inv;
+      }
     }
   }
   template <typename R>
   __device__ static R u(const BvpDev& b, R x, R y) {
     const R inv = R(1) / (R(2) * R(b.prob[2]));
-    return FrankeEval<R>((x - R(b.prob[0])) * inv + R(0.5), (y - R(b.prob[1])) * inv + R(0.5)).u();
+    return franke_value((x - R(b.prob[0])) * inv + R(0.5), (y - R(b.prob[1])) * inv + R(0.5));
   }
 };
 
@@ -489,12 +603,22 @@ struct RobinOf<4> {
   static constexpr bool value = true;
 };
 
+// What FP64 stepping need not compute for a problem: constant sigma, no drift
+// and no potential (then Y stays 1).
+template <int PROB>
+struct TraitsOf {
+  static constexpr bool const_sigma = PROB != 2 && PROB != 4;
+  static constexpr bool no_drift = PROB != 2 && PROB != 4;
+  static constexpr bool no_potential = PROB == 0 || PROB == 3 || PROB == 5;
+};
+
 // ---- the compiled problem functor sets --------------------------------------
 // Every BVP functor set the library compiles, indexed by FK_PROBLEM_*
 // (include/spac_fk.h).  To add one: write its Problem<N> (state, sigma_of,
 // step and u as above, all for both stepping types; psi and a RobinOf<N>
 // specialisation if it has reflecting sides; a DomainOf<N> specialisation if
-// its domain is a circle), give it FK_PROBLEM_ value N = kNumProblems and
+// its domain is a circle; a TraitsOf<N> specialisation if sigma, drift or
+// potential are not as the default says), give it FK_PROBLEM_ value N = kNumProblems and
 // raise kNumProblems.  with_problem then instantiates and dispatches every
 // kernel (paths, finalize, disk rows) for it; the registry accepts it and
 // checks its domain shape.

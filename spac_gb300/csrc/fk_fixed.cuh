@@ -1,0 +1,552 @@
+// 64-bit fixed-point building blocks of FP64 stepping.
+//
+// FP64 arithmetic runs at 1/64 of the FP32 rate on this part (two lanes per
+// SM and cycle: one FP64 warp instruction every 16 cycles), so a path step
+// written in FP64 is bound by that pipe alone: about 225 such instructions
+// per step for the Franke problem, 3,600 cycles, while the other pipes idle.
+// The functions here compute the step's transcendental and polynomial parts
+// on the integer pipes in 64-bit fixed point, at 52 to 60 fractional bits:
+// no operand, intermediate or result carries less precision than the FP64
+// forms they replace (errors are below, measured against 80-bit arithmetic
+// in tests/cpp/fixed_math_main.cpp).  A 64 x 64 product's upper half is three
+// 32 x 32 -> 64 multiply-adds, about 8 of the 64 issue slots that one FP64
+// instruction takes.
+//
+// The methods are the usual table-driven ones (P. T. P. Tang, ACM TOMS 1989
+// and 1990, for exp and log: a table at the leading bits and a short Taylor
+// polynomial for the rest), with exact integer argument reduction.  Tables
+// are built at compile time by integer arithmetic from a few mathematical
+// constants.
+//
+// Host and device give the same bits (the square root's seed excepted, whose
+// error the iteration removes).
+#pragma once
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define FX_FN __host__ __device__ __forceinline__
+#else
+#define FX_FN inline
+#endif
+
+namespace fk {
+namespace fx {
+
+typedef uint64_t u64;
+typedef int64_t i64;
+typedef uint32_t u32;
+
+// ------------------------------------------------------------ products -----
+FX_FN u32 mulhi32(u32 a, u32 b) { return static_cast<u32>((static_cast<u64>(a) * b) >> 32); }
+// (a b) >> 64 for a, b < 2^63, low by less than 2 units (the product of the
+// low words is dropped).
+FX_FN u64 mulhi(u64 a, u64 b) {
+  const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a), bh = static_cast<u32>(b >> 32), bl = static_cast<u32>(b);
+  u64 t = static_cast<u64>(ah) * bl;
+  t += static_cast<u64>(al) * bh;
+  return static_cast<u64>(ah) * bh + (t >> 32);
+}
+// (a b) >> S, 32 < S < 64, for a, b < 2^63 and a result below 2^64, low by less than 2 units.
+template <int S>
+FX_FN u64 mulshr(u64 a, u64 b) {
+  const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a), bh = static_cast<u32>(b >> 32), bl = static_cast<u32>(b);
+  u64 t = static_cast<u64>(ah) * bl + mulhi32(al, bl);
+  t += static_cast<u64>(al) * bh;
+  return ((static_cast<u64>(ah) * bh) << (64 - S)) + (t >> (S - 32));
+}
+// a^2 >> 63 for a < 2^63.5, low by less than 2 units.
+FX_FN u64 sqr63(u64 a) {
+  const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a);
+  return ((static_cast<u64>(ah) * ah) << 1) + ((static_cast<u64>(ah) * al + (mulhi32(al, al) >> 1)) >> 30);
+}
+// a^2 >> 64 for a < 2^63, low by less than 2 units.
+FX_FN u64 sqrhi(u64 a) {
+  const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a);
+  return static_cast<u64>(ah) * ah + ((static_cast<u64>(ah) * al) >> 31);
+}
+// Signed: (a b) >> 64 and (a b) >> S (32 < S < 64) for |a|, |b| < 2^62, low by less than 2 units.
+FX_FN i64 smulhi(i64 a, i64 b) {
+  const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
+  const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
+  const i64 t = ah * bl + al * bh;
+  return static_cast<i64>(ah) * bh + (t >> 32);
+}
+template <int S>
+FX_FN i64 smulshr(i64 a, i64 b) {
+  const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
+  const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
+  const i64 t = ah * bl + al * bh + static_cast<i64>(mulhi32(static_cast<u32>(a), static_cast<u32>(b)));
+  return static_cast<i64>(static_cast<u64>(static_cast<i64>(ah) * bh) << (64 - S)) + (t >> (S - 32));
+}
+FX_FN int clz64(u64 v) {
+#ifdef __CUDA_ARCH__
+  return __clzll(static_cast<long long>(v));
+#else
+  return v ? __builtin_clzll(v) : 64;
+#endif
+}
+
+// ------------------------------------------------------------- tables ------
+constexpr u64 kLn2_63 = 0x58B90BFBE8E7BCD6ull;  // ln 2 * 2^63
+constexpr u64 kLn2_59 = 0x058B90BFBE8E7BCDull;  // ln 2 * 2^59
+
+struct LogEntry {
+  u64 ln;   // -ln(c / 2^16) * 2^59
+  u64 c;    // reciprocal of the interval's middle, 16 bits
+};
+struct SinCosEntry {
+  u64 c, s;  // cos, sin of the cell's middle * 2^63
+};
+struct Tables {
+  u64 exp2[1024];       // 2^(j/1024) * 2^62
+  SinCosEntry sc[1024]; // angle (j + 1/2) / 4096 of a turn
+  LogEntry log[512];    // y in [1 + j/512, 1 + (j+1)/512)
+};
+
+// exact upper half of a 64 x 64 product (compile time)
+constexpr u64 cmulhi(u64 a, u64 b) {
+  const u64 ah = a >> 32, al = a & 0xffffffffu, bh = b >> 32, bl = b & 0xffffffffu;
+  const u64 m = ah * bl + ((al * bl) >> 32), n = al * bh + (m & 0xffffffffu);
+  return ah * bh + (m >> 32) + (n >> 32);
+}
+constexpr Tables make_tables() {
+  Tables t{};
+  // 2^(2^-i) * 2^63, i = 1 .. 10
+  constexpr u64 root[10] = {0xB504F333F9DE6484ull, 0x9837F0518DB8A96Full, 0x8B95C1E3EA8BD6E7ull, 0x85AAC367CC487B15ull,
+                            0x82CD8698AC2BA1D7ull, 0x8164D1F3BC030773ull, 0x80B1ED4FD999AB6Cull, 0x8058D7D2D5E5F6B1ull,
+                            0x802C6436D0E04F51ull, 0x8016302F17467628ull};
+  for (int j = 0; j < 1024; ++j) {
+    u64 v = 1ull << 63;  // Q1.63; each factor below 2 keeps the product below 2
+    for (int i = 0; i < 10; ++i)
+      if ((j >> (9 - i)) & 1) {
+        const u64 p = cmulhi(v, root[i]);  // Q2.62
+        v = (p << 1) | 1u;                 // (middle of the dropped bit)
+      }
+    t.exp2[j] = v >> 1;
+  }
+  // cos and sin of 2^-i of a turn * 2^64, i = 3 .. 13, then angle (2j + 1) / 8192 from its binary digits
+  constexpr u64 cr[11] = {0xB504F333F9DE6484ull, 0xEC835E79946A3145ull, 0xFB14BE7FBAE58156ull, 0xFEC46D1E89292CF0ull,
+                            0xFFB10F1BCB6BEF1Dull, 0xFFEC4304266865D9ull, 0xFFFB10B4DC96DABCull, 0xFFFEC42C7454926Bull,
+                            0xFFFFB10B10E80E95ull, 0xFFFFEC42C3773236ull, 0xFFFFFB10B0D19F76ull};
+  constexpr u64 sr[11] = {0xB504F333F9DE6484ull, 0x61F78A9ABAA58B47ull, 0x31F17078D34C156Dull, 0x1917A6BC29B42BE2ull,
+                            0x0C8FB2F886EC09F3ull, 0x0648557DE8D99F7Eull, 0x03243A3F9BD8F08Dull, 0x01921F0FE6700712ull,
+                            0x00C90FC5F66525D2ull, 0x006487EABB991CB6ull, 0x003243F655D966C1ull};
+  for (int j = 0; j < 1024; ++j) {
+    const int a = 2 * j + 1;  // of 8192ths of a turn, below 2048
+    u64 c = 0, s = 0;
+    bool one = true;  // (cos 0 = 1 does not fit 64 fractional bits)
+    for (int i = 0; i < 11; ++i)
+      if ((a >> (10 - i)) & 1) {
+        if (one) {
+          c = cr[i];
+          s = sr[i];
+          one = false;
+        } else {
+          const u64 cn = cmulhi(c, cr[i]) - cmulhi(s, sr[i]);
+          s = cmulhi(s, cr[i]) + cmulhi(c, sr[i]);
+          c = cn;
+        }
+      }
+    t.sc[j].c = c >> 1;
+    t.sc[j].s = s >> 1;
+  }
+  for (int j = 0; j < 512; ++j) {
+    const u64 d = 1025 + 2 * static_cast<u64>(j);  // middle of the interval: d / 1024
+    u64 c = ((1ull << 27) / d + 1) >> 1;           // 2^16 / (d / 1024), rounded
+    if (j == 511) c = 1ull << 15;                  // exactly 1/2: -ln u is exact near u = 1
+    // -ln(c / 2^16) = 2 atanh((2^16 - c) / (2^16 + c)), series in 2^64
+    const u64 num = 65536 - c, den = 65536 + c;
+    u64 x = 0, r = num;
+    for (int b = 0; b < 64; ++b) {
+      r <<= 1;
+      x <<= 1;
+      if (r >= den) {
+        r -= den;
+        x |= 1;
+      }
+    }
+    const u64 x2 = cmulhi(x, x);
+    u64 p = x, sum = 0;
+    for (int k = 1; k < 60 && p; k += 2) {
+      sum += p / k;
+      p = cmulhi(p, x2);
+    }
+    t.log[j].ln = j == 511 ? kLn2_59 : (sum >> 4) + ((sum >> 3) & 1);  // 2 sum 2^-64 in 2^-59
+    t.log[j].c = c;
+  }
+  return t;
+}
+#ifdef __CUDACC__
+static __device__ const Tables kTablesDev = make_tables();
+#endif
+#ifndef __CUDA_ARCH__
+static constexpr Tables kTablesHost = make_tables();
+#endif
+FX_FN const Tables& tables() {
+#ifdef __CUDA_ARCH__
+  return kTablesDev;
+#else
+  return kTablesHost;
+#endif
+}
+
+// ------------------------------------------------- conversions -------------
+FX_FN u64 bits_of(double v) {
+#ifdef __CUDA_ARCH__
+  return static_cast<u64>(__double_as_longlong(v));
+#else
+  u64 u;
+  std::memcpy(&u, &v, 8);
+  return u;
+#endif
+}
+FX_FN double from_bits(u64 u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double(static_cast<long long>(u));
+#else
+  double v;
+  std::memcpy(&v, &u, 8);
+  return v;
+#endif
+}
+// mag 2^e2 with the given sign (0 or 1), rounded to nearest, on the integer
+// pipes; mag = 0 gives 2^(e2 - 1).
+FX_FN double to_double(u64 mag, u32 sign, int e2) {
+  const int n = clz64(mag | 1);
+  const u64 m = mag << n;
+  const u64 b = (static_cast<u64>(1085 - n + e2) << 52) + (m >> 11) + ((m >> 10) & 1);
+  return from_bits(b | (static_cast<u64>(sign) << 63));
+}
+FX_FN double to_double(i64 v, int e2) {
+  const i64 s = v >> 63;
+  return to_double(static_cast<u64>((v ^ s) - s), static_cast<u32>(s) & 1u, e2);
+}
+
+// -------------------------------------------------------------- exp2 -------
+// 2^(f / 2^54) for the fraction f in [0, 2^54), times 2^62; relative error
+// below 2^-58 (the table's, the truncated products' and the dropped z^5 term).
+FX_FN u64 exp2_frac(u64 f) {
+  const u32 j = static_cast<u32>(f >> 44);
+  // z = (f mod 2^44) 2^-54 ln 2 < 6.8e-4, as z 2^64; e^z - 1 by its series
+  const u64 z = mulhi((f & ((1ull << 44) - 1)) << 11, kLn2_63);
+  const u32 zh = static_cast<u32>(z >> 22), zl = static_cast<u32>(z) & 0x3fffffu;
+  const u64 z2 = ((static_cast<u64>(zh) * zh) >> 21) + ((static_cast<u64>(zh) * zl) >> 42);  // z^2 / 2
+  const u32 z3 = mulhi32(mulhi32(static_cast<u32>(z2 >> 10), 0x55555556u), zh);              // z^3 / 6
+  const u32 z4 = mulhi32(z3, zh) >> 12;                                                      // z^4 / 24
+#ifdef __CUDA_ARCH__
+  const u64 T = __ldg(reinterpret_cast<const unsigned long long*>(&kTablesDev.exp2[j]));
+#else
+  const u64 T = tables().exp2[j];
+#endif
+  return T + mulhi(T, z + z2 + (z3 + z4));
+}
+// 2^(q 2^-54) 2^F for q >= -2^62 and a result below 2^63 (truncated).
+template <int F>
+FX_FN u64 exp2_fx(i64 q) {
+  const int sh = 62 - F - static_cast<int>(q >> 54);
+  return exp2_frac(static_cast<u64>(q) & ((1ull << 54) - 1)) >> (sh < 63 ? sh : 63);
+}
+// e^v for |v| < 256, relative error below 1.1 2^-53 (the rounding of the result and
+// 2^-54 from the exponent's 54 fractional bits).
+FX_FN double exp_core(double v) {
+  const u64 b = bits_of(v);
+  const int e = static_cast<int>(b >> 52) & 0x7ff;
+  const u64 m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;  // |v| = m 2^(e - 1085), m < 2^63
+  const int s = 1031 - e;                                                 // > 0 for |v| < 256: |v| 2^54 = m >> s
+  const u64 V = s < 63 ? m >> s : 0;
+  // t = |v| log2(e) = V + 0.44 V
+  i64 q = static_cast<i64>(V + mulhi(V, 0x71547652B82FE177ull) + 1);
+  if (b >> 63) q = -q;
+  const u64 M = exp2_frac(static_cast<u64>(q) & ((1ull << 54) - 1));
+  return from_bits((static_cast<u64>(1022 + static_cast<int>(q >> 54)) << 52) + (M >> 10) + ((M >> 9) & 1));
+}
+
+// --------------------------------------------------------- square root -----
+// sqrt(A 2^e) for A in [2^62, 2^64) and even e: root 2^61 sqrt(A 2^-64) (in
+// [2^60, 2^61]), the value being root 2^((e + 64) / 2 - 61); relative error
+// below 2^-57.  Seed y ~ (A 2^-64)^-1/2 of 22 bits, h = 1 - a y^2 exactly,
+// sqrt(a) = a y (1 + h/2 + 3 h^2 / 8 + O(2^-63)).
+FX_FN u64 sqrt_core(u64 A) {
+  const float af = static_cast<float>(static_cast<u32>(A >> 40)) * 5.9604644775390625e-8f;
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(af));
+#else
+  float y = 1.0f / std::sqrt(af);
+#endif
+  y = y < 1.99999988f ? y : 1.99999988f;
+  y = y > 1.0f ? y : 1.0f;
+#ifdef __CUDA_ARCH__
+  const u32 yb = static_cast<u32>(__float_as_uint(y));
+#else
+  u32 yb;
+  std::memcpy(&yb, &y, 4);
+#endif
+  const u32 Y = (yb & 0x7fffffu) | 0x800000u;  // y 2^23
+  const u64 A1 = A >> 1;                       // a 2^63
+  const i64 h = static_cast<i64>((1ull << 60) - mulhi(A1, (static_cast<u64>(Y) * Y) << 15));  // (1 - a y^2) 2^60
+  const u64 g = mulhi(A1, static_cast<u64>(Y) << 39);                                         // a y 2^61
+  const int hh = static_cast<int>(h >> 9);
+  const i64 corr = (h >> 1) + 3 * static_cast<i64>((static_cast<u64>(static_cast<i64>(hh) * hh)) >> 45);  // (h/2 + 3h^2/8) 2^60
+  const i64 sg = corr >> 63;
+  const u64 d = mulshr<60>(g, static_cast<u64>((corr ^ sg) - sg));
+  return g + static_cast<u64>((static_cast<i64>(d) ^ sg) - sg);
+}
+// sqrt(L 2^e) for L > 0: a root in [2^60, 2^61] and its exponent.
+FX_FN u64 sqrt_norm(u64 L, int e, int& e_out) {
+  const int n = clz64(L);
+  u64 A = L << n;
+  e -= n;
+  if (e & 1) {
+    A >>= 1;
+    e += 1;
+  }
+  e_out = ((e + 64) >> 1) - 61;
+  return sqrt_core(A);
+}
+
+// -------------------------------------------------- normal pair -------------
+// l = -ln((a + 1/2) 2^-32) as l 2^59 (e = -58) or, in the last table cell
+// before u = 1, l 2^69 (e = -68); absolute error below 2^-55, there 2^-66.
+// Exact argument reduction: u = y 2^(30-n), y c - 1 an integer multiple of 2^-48.
+FX_FN u64 neg_log(u32 a, int& e) {
+  const u64 m = (static_cast<u64>(a) << 1) | 1u;
+  const int n = clz64(m);
+  const u64 Y = m << n;  // y 2^63, y in [1, 2)
+  const u32 j = static_cast<u32>(Y >> 54) & 511u;
+#ifdef __CUDA_ARCH__
+  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.log[j]));
+  const u64 ln = t.x, c = t.y;
+#else
+  const u64 ln = tables().log[j].ln, c = tables().log[j].c;
+#endif
+  const i64 r = static_cast<i64>((Y >> 31) * c - (1ull << 48));  // (y c - 1) 2^48, |r| < 2^38.1
+  const i64 sg = r >> 63;
+  const u64 A = static_cast<u64>((r ^ sg) - sg) << 24;  // |r| 2^72
+  const u64 r2 = sqrhi(A);                              // r^2 2^80
+  const u32 rh = static_cast<u32>(A >> 32), q = static_cast<u32>(r2 >> 29);  // |r| 2^40, r^2 2^51
+  const u32 r4 = mulhi32(q, q);                                              // r^4 2^70
+  const u64 odd = (A >> 3) + ((static_cast<u64>(mulhi32(q, 0x55555555u)) * rh) >> 22) +
+                  (mulhi32(mulhi32(r4, rh), 0x33333334u) >> 9);  // |r| + |r|^3/3 + |r|^5/5
+  const u64 even = (r2 >> 12) + (r4 >> 3);                       // r^2/2 + r^4/4
+  const i64 l1p = ((static_cast<i64>(odd) ^ sg) - sg) - static_cast<i64>(even);  // log1p(r) 2^69
+  const u64 base = static_cast<u64>(n - 30) * kLn2_59 - ln;
+  e = base ? -58 : -68;
+  return base ? base - static_cast<u64>(l1p >> 10) : static_cast<u64>(-l1p);
+}
+
+// cos and sin of the angle b + 1/2 (of 2^32) within its quadrant, times 2^63;
+// absolute error below 2^-58 (the dropped theta^5 / 120 term is 2^-58.6).
+FX_FN void sincos_quadrant(u32 b, u64& cs, u64& sn) {
+  const u32 j = (b >> 20) & 1023u;
+#ifdef __CUDA_ARCH__
+  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.sc[j]));
+  const u64 C = t.x, S = t.y;
+#else
+  const u64 C = tables().sc[j].c, S = tables().sc[j].s;
+#endif
+  // theta = 2 pi D 2^-33 from the cell's middle, |D| < 2^20, odd
+  const int D = static_cast<int>(2u * (b & 0xfffffu) + 1u) - (1 << 20);
+  const int sg = D >> 31;
+  const u32 Da = static_cast<u32>((D ^ sg) - sg);
+  const u64 hq = mulhi(static_cast<u64>(Da) * Da << 23, 0x4EF4F326F9177969ull);  // theta^2 / 2 * 2^83
+  const u32 q = static_cast<u32>(hq >> 30);                                      // theta^2 / 2 * 2^53
+  const u64 th = mulhi(static_cast<u64>(Da) << 43, 0x6487ED5110B4611Aull);       // theta 2^72 (2 pi 2^60)
+  const u64 c1 = (hq >> 20) - (mulhi32(mulhi32(q, q), 0x2AAAAAABu) >> 11);       // (1 - cos theta) 2^63
+  const u64 s1 = (th >> 9) - mulhi32(static_cast<u32>(th >> 30), mulhi32(q, 0x55555556u));  // sin |theta| 2^63
+  const u64 cc = mulhi(C, c1 << 1), ss = mulhi(S, s1 << 1), sc = mulhi(S, c1 << 1), csn = mulhi(C, s1 << 1);
+  const u64 m = static_cast<u64>(static_cast<i64>(sg));
+  cs = C - cc - ((ss ^ m) - m);
+  sn = S - sc + ((csn ^ m) - m);
+}
+
+// Box-Muller pair sqrt(-2 ln u1) (cos, sin)(2 pi u2), u = (word + 1/2) 2^-32:
+// absolute error below 2^-56 for |z| of order 1.
+FX_FN void normal_pair(u32 a, u32 b, double& z0, double& z1) {
+  int el, e;
+  const u64 l = neg_log(a, el);
+  const u64 rad = sqrt_norm(l, el, e);  // sqrt(2 l) = rad 2^e, rad in [2^60, 2^61]
+  u64 c, s;
+  sincos_quadrant(b, c, s);
+  const u32 quad = b >> 30;
+  const u64 pc = (quad & 1u) ? s : c, ps = (quad & 1u) ? c : s;
+  z0 = to_double(mulhi(rad, pc), (quad ^ (quad >> 1)) & 1u, e + 1);
+  z1 = to_double(mulhi(rad, ps), quad >> 1, e + 1);
+}
+
+// ------------------------------------------------------ Franke function ----
+// Positions are 2^-59 units.  In [-3/8, 11/8)^2, which holds the unit square
+// and the serial driver's domain, the sums of squares stay below 256 and the
+// slowest exponential above 6e-3, so absolute errors of 2^-50 are relative
+// ones of the same order; elsewhere the FP64 forms run.
+FX_FN bool to_pos(double v, i64& p) {
+  const u64 b = bits_of(v);
+  const int e = static_cast<int>(b >> 52) & 0x7ff;
+  const u64 m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;  // |v| = m 2^(e - 1085)
+  int s = 1026 - e;
+  const bool small = s >= 3;  // |v| < 2
+  s = small ? (s < 63 ? s : 63) : 3;
+  const i64 sg = static_cast<i64>(b) >> 63;
+  p = (static_cast<i64>(m >> s) ^ sg) - sg;
+  // -3/8 <= p 2^-59 < 11/8
+  return small && static_cast<u32>(p >> 32) + 0x03000000u < 0x0E000000u;
+}
+constexpr u64 kOne55 = 1ull << 55;
+constexpr u64 kLog2e_4 = 0x5C551D94AE0BF85Eull;  // log2(e) / 4 * 2^64
+
+// Squares (2^-55 units) and base-2 exponents (2^-54) of the four exponentials.
+// One square per coordinate: (9x - k)^2 = (9x)^2 - 2k (9x) + k^2, exact sums.
+struct FrankeArgs {
+  i64 X9, Y9;       // 9x, 9y (2^-59)
+  u64 Gx, Gy;       // (9x)^2, (9y)^2
+  u64 s1, s3, s4;   // a^2 + b^2, p^2 + q^2, r^2 + t^2
+  u64 c2;           // (9x + 1)^2
+  i64 t1, t2, t3, t4;  // e_i = 2^-t_i
+};
+FX_FN u64 abs64(i64 v) {
+  const i64 s = v >> 63;
+  return static_cast<u64>((v ^ s) - s);
+}
+FX_FN void franke_args(i64 X, i64 Y, FrankeArgs& f) {
+  f.X9 = 9 * X;
+  f.Y9 = 9 * Y;
+  f.Gx = sqr63(abs64(f.X9)) + 1;
+  f.Gy = sqr63(abs64(f.Y9)) + 1;
+  const i64 S = static_cast<i64>(f.Gx + f.Gy + 2);  // (the 2: no sum below falls under zero by rounding)
+  const i64 xq = f.X9 >> 2, xe = f.X9 >> 3, yq = f.Y9 >> 2, ye = f.Y9 >> 3;
+  f.s1 = static_cast<u64>(S - xq - yq) + 8 * kOne55;
+  f.s3 = static_cast<u64>(S - (f.X9 - xe) - (yq + ye)) + 58 * kOne55;
+  f.s4 = static_cast<u64>(S - (f.X9 >> 1) - (f.Y9 - ye)) + 65 * kOne55;
+  f.c2 = f.Gx + 2 + static_cast<u64>(xe) + kOne55;
+  f.t1 = static_cast<i64>((mulhi(f.s1, kLog2e_4) + 1) >> 1);
+  f.t3 = static_cast<i64>((mulhi(f.s3, kLog2e_4) + 1) >> 1);
+  f.t4 = static_cast<i64>((f.s4 + mulhi(f.s4, 0x71547652B82FE177ull) + 1) >> 1);
+  // (9x + 1)^2 / 49 + (9y + 5) / 10 - 4 / 10, times log2(e)
+  const u64 d = static_cast<u64>(f.Y9 >> 1) + (5ull << 58);
+  f.t2 = static_cast<i64>((mulhi(f.c2, 0x07898F79D9F68737ull) >> 1) + (mulhi(d, 0x24EED8A1DF37FCF2ull) >> 4) - 0x0024EED8A1DF37FCull);
+}
+// Laplacian of the Franke function, 2^-54 units; each coefficient is folded
+// into its exponential's exponent (log2 of 243/16, 486/4802, 81/8, 324/5):
+// lap = 243/16 (s1 - 4) e1 + 81/8 (s3 - 4) e3 - 324/5 (s4 - 1) e4 + 486/4802 (c2 - 18.4975) e2
+FX_FN i64 franke_lap(const FrankeArgs& f) {
+  const u64 E1 = exp2_fx<59>(70703136514952234ll - f.t1), E3 = exp2_fx<59>(60165388913858184ll - f.t3);
+  const u64 E4 = exp2_fx<56>(108409243449604861ll - f.t4), E2 = exp2_fx<62>(-59530510741125490ll - f.t2);
+  i64 l = static_cast<i64>(mulshr<60>(f.s1, E1)) - static_cast<i64>(E1 >> 3);
+  l += static_cast<i64>(mulshr<60>(f.s3, E3)) - static_cast<i64>(E3 >> 3);
+  l -= static_cast<i64>(mulshr<57>(f.s4, E4)) - static_cast<i64>(E4 >> 2);
+  l += static_cast<i64>(mulshr<63>(f.c2, E2)) - static_cast<i64>(mulhi(E2, 0x127F5C28F5C28F5Cull));
+  return l;
+}
+// b1 = 3/4 e1, b2 = 3/4 e2, b3 = e3 / 2, b4 = e4 / 5, 2^-60 units: u = b1 + b2 + b3 - b4
+struct FrankeTerms {
+  u64 b1, b2, b3, b4;
+};
+FX_FN void franke_terms(const FrankeArgs& f, FrankeTerms& b) {
+  b.b1 = exp2_fx<60>(-7476650908387934ll - f.t1);
+  b.b2 = exp2_fx<60>(-7476650908387934ll - f.t2);
+  b.b3 = exp2_fx<59>(-f.t3);
+  b.b4 = exp2_fx<60>(-41828138011663243ll - f.t4);
+}
+FX_FN i64 franke_u(const FrankeTerms& b) { return static_cast<i64>(b.b1 + b.b2 + b.b3 - b.b4); }
+// u_x and u_y, 2^-58 units (g = 18/49):
+// u_x = 9x (-9/2 (b1 + b3) - g b2 + 18 b4) + 9 b1 - g b2 + 63/2 b3 - 72 b4
+// u_y = 9y (-9/2 (b1 + b3) + 18 b4) + 9 b1 - 9/10 b2 + 27/2 b3 - 126 b4
+FX_FN void franke_grad(const FrankeArgs& f, const FrankeTerms& b, i64& ux, i64& uy) {
+  const u64 gb = mulhi(b.b2, 0x2F05397829CBC14Full);  // g b2, 2^-59
+  const i64 wy = static_cast<i64>(9 * b.b4) - static_cast<i64>((9 * ((b.b1 + b.b3) >> 1)) >> 1);  // 2^-59
+  const i64 wx = wy - static_cast<i64>(gb);
+  const u64 v = 2 * b.b1 + (b.b1 >> 2);
+  const u64 vx = v - (gb >> 1) + 8 * b.b3 - (b.b3 >> 3) - 18 * b.b4;
+  const u64 vy = v - mulhi(b.b2, 0x399999999999999Aull) + 3 * b.b3 + ((3 * b.b3) >> 3) - 32 * b.b4 + (b.b4 >> 1);
+  ux = static_cast<i64>((static_cast<u64>(smulhi(f.X9 >> 1, wx)) << 5) + vx);
+  uy = static_cast<i64>((static_cast<u64>(smulhi(f.Y9 >> 1, wy)) << 5) + vy);
+}
+// Laplacian from the same terms, 2^-54 units:
+// 81/4 ((s1 - 4) b1 + (s3 - 4) b3) - 324 (s4 - 1) b4 + (g^2 c2 - 9 g + 81/100) b2
+FX_FN i64 franke_lap_terms(const FrankeArgs& f, const FrankeTerms& b) {
+  const i64 p = static_cast<i64>(mulshr<57>(f.s1, b.b1) - b.b1) + static_cast<i64>(mulshr<57>(f.s3, b.b3) - b.b3);  // 2^-58
+  const i64 p4 = static_cast<i64>(mulshr<55>(f.s4, b.b4) - b.b4);                                                  // 2^-60
+  const i64 p2 = static_cast<i64>(mulshr<60>(mulhi(f.c2, 0x228BACD5ABC4B7D1ull), b.b2)) -
+                 static_cast<i64>(mulhi(b.b2, 0x13F80F0BE96E21DBull));                                             // 2^-55
+  return (2 * p + (p >> 1) + (p >> 5) - ((20 * p4 + (p4 >> 2)) >> 1) + p2) >> 1;
+}
+
+// -------------------------------------- the anisotropic problem's factors ----
+// sin(2 pi x), 2^-63 units and its sign; x in 2^-59 units of a turn.
+FX_FN u64 sin_turn(i64 X, u32& neg) {
+  const u32 quad = static_cast<u32>(X >> 57) & 3u, j = static_cast<u32>(X >> 47) & 1023u;
+#ifdef __CUDA_ARCH__
+  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.sc[j]));
+  const u64 C = t.x, S = t.y;
+#else
+  const u64 C = tables().sc[j].c, S = tables().sc[j].s;
+#endif
+  const i64 D = (X & ((1ll << 47) - 1)) - (1ll << 46);  // theta = 2 pi D 2^-59 from the cell's middle
+  const i64 sg = D >> 63;
+  const u64 th = mulhi(static_cast<u64>((D ^ sg) - sg) << 17, 0x6487ED5110B4611Aull);  // theta 2^72
+  const u64 hq = sqrhi(th) << 2;                                                       // theta^2 / 2 * 2^83
+  const u32 q = static_cast<u32>(hq >> 30);
+  const u64 c1 = (hq >> 20) - (mulhi32(mulhi32(q, q), 0x2AAAAAABu) >> 11);
+  const u64 s1 = (th >> 9) - mulhi32(static_cast<u32>(th >> 30), mulhi32(q, 0x55555556u));
+  const u64 P = (quad & 1u) ? C : S, Q = (quad & 1u) ? S : C;
+  const u64 m = static_cast<u64>((quad & 1u) ? ~sg : sg);
+  neg = quad >> 1;
+  return P - mulhi(P, c1 << 1) + ((mulhi(Q, s1 << 1) ^ m) - m);
+}
+// a = 1 + sin(2 pi x) sin(2 pi y) / 2, 2^-62 units
+FX_FN u64 aniso_a(i64 X, i64 Y) {
+  u32 nx, ny;
+  const u64 sx = sin_turn(X, nx), sy = sin_turn(Y, ny);
+  const u64 p = mulhi(sx, sy) >> 1;
+  const u64 m = 0ull - static_cast<u64>(nx ^ ny);
+  return (1ull << 62) + ((p ^ m) - m);
+}
+// v 2^62 of a double v in [2^-10, 2)
+FX_FN u64 a_bits(double v) {
+  const u64 b = bits_of(v);
+  return ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10 >> ((1023 - static_cast<int>(b >> 52)) & 63);
+}
+FX_FN double aniso_sigma(u64 a62) {  // sqrt(2 a)
+  int e;
+  const u64 r = sqrt_norm(a62, -61, e);
+  return to_double(r, 0u, e);
+}
+// The anisotropic problem at a point: source f (2^-51 units) of
+// u = F q, q = 1 + xy, F the Franke function:
+//   f = -(q (a lap F + b . grad F + c F) + 2 a (F_x y + F_y x) + F (y^2 - x^2 + (x - y) / 2)),
+// b = (y - 1/2, 1/2 - x), c = -(1 + x^2 + y^2); and -c (2^-54 units).
+struct AnisoOut {
+  i64 f;
+  u64 mc;
+  i64 F, Fx, Fy, q;  // 2^-60, 2^-58, 2^-58, 2^-60 units
+};
+FX_FN void aniso_step(i64 X, i64 Y, u64 a62, AnisoOut& o) {
+  FrankeArgs f;
+  FrankeTerms b;
+  franke_args(X, Y, f);
+  franke_terms(f, b);
+  o.F = franke_u(b);
+  franke_grad(f, b, o.Fx, o.Fy);
+  const i64 lap = franke_lap_terms(f, b);
+  const i64 X61 = X << 2, Y61 = Y << 2, a61 = static_cast<i64>(a62 >> 1);
+  o.q = (1ll << 60) + (smulhi(X61, Y61) << 2);
+  o.mc = (kOne55 + mulhi(f.Gx + f.Gy, 0x0329161F9ADD3C0Dull)) >> 1;
+  const i64 adv = smulhi(Y61 - (1ll << 60), o.Fx) + smulhi((1ll << 60) - X61, o.Fy) - smulhi(static_cast<i64>(o.mc << 5), o.F);  // 2^-55
+  const i64 inner = (smulhi(lap, a61) << 2) + (adv >> 2);                  // 2^-53
+  const i64 t1 = smulshr<62>(inner, o.q);                                  // 2^-51
+  const i64 g = smulhi(o.Fx, Y61) + smulhi(o.Fy, X61);                     // 2^-55
+  const i64 t2 = smulhi(g << 1, a61) >> 1;                                 // 2 a g, 2^-51
+  const i64 h = smulhi(static_cast<i64>(f.Gy - f.Gx) >> 1, 0x0329161F9ADD3C0Dll) + ((X - Y) >> 6);  // 2^-54
+  const i64 t3 = smulhi(o.F, h << 6) >> 5;                                 // 2^-51
+  o.f = -(t1 + t2 + t3);
+}
+// grad u = grad F q + F (y, x), 2^-54 units
+FX_FN void aniso_grad(i64 X, i64 Y, const AnisoOut& o, i64& ux, i64& uy) {
+  ux = smulhi(o.Fx, o.q) + (smulhi(o.F, Y << 2) >> 3);
+  uy = smulhi(o.Fy, o.q) + (smulhi(o.F, X << 2) >> 3);
+}
+
+}  // namespace fx
+}  // namespace fk

@@ -649,6 +649,23 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     }
     const R st0 = Problem<PROB>::template state<R>(bvp, x0, y0);  // sigma state at the start point
     const R sg0 = Problem<PROB>::template sigma_of<R>(st0);
+    // FP64 stepping (kLean): the exit test of Dentro with few FP64
+    // instructions, which bound it (one takes 64 issue slots here).  A path
+    // goes on iff every boundary's signed distance is below the (negative)
+    // threshold, so the distances alone are formed, from centres and half
+    // sides kept here; a circle's test compares squared radii, without the
+    // square root.  Dentro's choice of boundary, projection and normal follow
+    // only when some lane of the warp stops.
+    constexpr bool kLean = std::is_same<R, double>::value && !RobinOf<PROB>::value;
+    R dcx = R(0), dcy = R(0), dhx = R(0), dhy = R(0), scx = R(0), scy = R(0), shx = R(0), shy = R(0);
+    if constexpr (kLean) {
+      if constexpr (DomainOf<PROB>::shape == 0) {
+        dcx = R(0.5) * (d0 + d2); dcy = R(0.5) * (d1 + d3); dhx = d2 - dcx; dhy = d3 - dcy;
+      }
+      if (!sub_circle) {
+        scx = R(0.5) * (s0 + s2); scy = R(0.5) * (s1 + s3); shx = s2 - scx; shy = s3 - scy;
+      }
+    }
     // Reflecting sides (FK_PROBLEM_ROBIN), only where the domain can win
     // Dentro's comparison.
     int rmask = 0;
@@ -844,8 +861,26 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         const uint32_t wa = r.x, wb = r.y;
         R z0, z1;
         box_muller(wa, wb, z0, z1);
+        if constexpr (kLean) {
+          // the Euler step with the terms that are zero for the problem left out
+          const R sh = co.s * sqrth;
+          Z += TraitsOf<PROB>::no_potential ? co.f * h : (co.f * Y) * h;
+          if (cv) {
+            const R dWx = sqrth * z0, dWy = sqrth * z1;
+            const R F = co.Fx * dWx + co.Fy * dWy;
+            xi += TraitsOf<PROB>::no_potential ? F : Y * F;
+          }
+          if constexpr (!TraitsOf<PROB>::no_potential) Y += (co.c * Y) * h;
+          if constexpr (!TraitsOf<PROB>::no_drift) {
+            x += co.bx * h;
+            y += co.by * h;
+          }
+          x += sh * z0;
+          y += sh * z1;
+        }
         const R dWx = sqrth * z0, dWy = sqrth * z1;
-        if constexpr (RobinOf<PROB>::value) {
+        if constexpr (kLean) {
+        } else if constexpr (RobinOf<PROB>::value) {
           // ---- Paso_Reflejante (FeynmanKacSolver.cpp:19-67) on reflecting sides
           R xn = x + (co.bx * h + co.s * dWx), yn = y + (co.by * h + co.s * dWy);
           R lt[4] = {R(0), R(0), R(0), R(0)};  // local time pushed back through each side
@@ -919,6 +954,30 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         }
         ++k;
         // ---- exit rule (Dentro, FeynmanKacSolver.cpp:68-106)
+        if constexpr (kLean) {
+          if constexpr (!TraitsOf<PROB>::const_sigma) {
+            st = Problem<PROB>::template state<R>(bvp, x, y);
+            sgc = Problem<PROB>::template sigma_of<R>(st);
+          }
+          const R thr = R(kGobet) * (sgc * sqrth);
+          // d < thr < 0 of a rectangle: the larger of two negative offsets, as integers
+          auto rect_in = [&](R cx, R cy, R hx, R hy) {
+            const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
+            // (a negative double grows as its bits fall; a non-negative or NaN offset fails the comparison)
+            return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
+          };
+          auto circle_in = [&](R r0, R cx, R cy) {  // |x - c|, at least 5e-4, below r0 + thr
+            const R nx = x - cx, ny = y - cy, rho = r0 + thr;
+            return rho > R(5e-4) && nx * nx + ny * ny < rho * rho;
+          };
+          bool in = true;
+          if (dom_can_win)
+            in = DomainOf<PROB>::shape == 1 ? circle_in(d0, d1, d2) : rect_in(dcx, dcy, dhx, dhy);
+          if (has_sub) in = in && (sub_circle ? circle_in(s0, s1, s2) : rect_in(scx, scy, shx, shy));
+          capped = k >= a.max_steps;
+          exits = !in || capped;
+        }
+        if (!kLean || exits) {
         Bnd<R> w;
         if (dom_can_win) {
           w = (DomainOf<PROB>::shape == 1) ? circle_dist<R>(x, y, d0, d1, d2) : rect_dist<R>(x, y, d0, d1, d2, d3);
@@ -930,6 +989,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           w = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
           dom_wins = false;
         }
+        if constexpr (!kLean) {
         // sigma at the new point (kept for the next step) or at the
         // projection: one evaluation at the selected point, no divergence
         const bool inside = w.d < R(0);
@@ -990,8 +1050,10 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
             sgc = Problem<PROB>::template sigma_of<R>(st);
           }
         }
+        }
         ex = w.ex;
         ey = w.ey;
+        }
       }
       // ---- queue the exits; the exiting lanes start their next path at once
       const unsigned em = __ballot_sync(kFull, exits);

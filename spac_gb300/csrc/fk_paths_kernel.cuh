@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     // the item's BVP (independent problems of one functor share a launch; the
     // control variate is the item's own, so learned-CV items and their plain
     // fallback can share one launch)
-    const BvpDev& bvp = a.bvp[itg.bvp];
+    const BvpDev bvp = a.bvp[itg.bvp];  // (a copy: the problem parameters are converted once per chunk, not per step)
     const bool cv_exact = CV && bvp.cv == 1;                // F from the problem functor
     const bool cv_table = CV && a.cv == 2 && bvp.cv == 2;   // F from the learned gradient table
     const bool cv = cv_exact || cv_table;             // any control term

@@ -7,6 +7,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/spac_fk.h"
@@ -150,13 +151,14 @@ struct fk_ctx {
   std::vector<std::unique_ptr<fk::Mesh>> meshes;
   std::vector<std::unique_ptr<fk::Mlp>> mlps;
   // workspace
-  fk::DBuf w_items, w_chunks, w_stats, w_acc, w_queue, w_gout, w_bout, w_sout, w_val, w_B, w_goff, w_row, w_tmp;
+  fk::DBuf w_items, w_chunks, w_stats, w_acc, w_queue, w_gout, w_bout, w_sout, w_val, w_B, w_goff, w_row, w_tmp, w_first;
   fk::DBuf w_dgrid, w_dcbar, w_dvar, w_dminv, w_dz, w_dG, w_dB, w_dflags;
   fk::DiskBufs w_disk;
-  fk::HBuf h_items, h_chunks, h_goff, h_stats, h_queue;  // pinned staging of the per-call transfers
+  fk::HBuf h_items, h_chunks, h_goff, h_stats, h_queue, h_first;  // pinned staging of the per-call transfers
   std::vector<fk::ItemDev> tmp_items;            // host scratch kept across calls
   std::vector<fk::ChunkDev> tmp_chunks, tmp_chunks2;
-  std::vector<unsigned> tmp_count;
+  std::vector<unsigned> tmp_count, tmp_cls;
+  std::vector<int> tmp_first;
 };
 
 namespace {
@@ -515,6 +517,90 @@ int finish_run(fk_ctx* ctx, RunOut& out) {
   return FK_OK;
 }
 
+// Groups the chunks of a streaming launch into classes of equal constants
+// (stencil, or for point solves BVP and step size), in the order of the
+// classes' first items and otherwise as they were; `first` gets the classes'
+// bounds.  More than kMaxClasses classes stay one list: a warp at its end
+// looks into every class once, and with so many each holds few chunks.
+constexpr unsigned kMaxClasses = 256;
+void group_chunks(fk_ctx* ctx, const std::vector<fk::ItemDev>& it, std::vector<fk::ChunkDev>& chunks, int kind,
+                  std::vector<int>& first) {
+  first.clear();
+  if (chunks.size() < 2) return;
+  std::vector<unsigned>& cls = ctx->tmp_cls;  // per item
+  cls.resize(it.size());
+  unsigned n = 0;
+  std::unordered_map<unsigned long long, unsigned> ids;
+  for (size_t i = 0; i < it.size(); ++i) {
+    const fk::ItemDev& x = it[i];
+    if (i > 0 && x.stencil == it[i - 1].stencil && x.bvp == it[i - 1].bvp && x.h == it[i - 1].h) {
+      cls[i] = cls[i - 1];
+      continue;
+    }
+    unsigned long long b;
+    std::memcpy(&b, &x.h, 8);
+    b = b * 0x9E3779B97F4A7C15ull + static_cast<unsigned>(x.bvp);
+    cls[i] = ids.emplace(b * 0x9E3779B97F4A7C15ull + static_cast<unsigned>(x.stencil), n).first->second;
+    n = std::max(n, cls[i] + 1);
+    if (n > kMaxClasses) return;
+  }
+  if (n < 2) return;
+  first.assign(n + 1, 0);
+  for (const fk::ChunkDev& c : chunks) ++first[cls[c.item] + 1];
+  for (unsigned l = 1; l <= n; ++l) first[l] += first[l - 1];
+  std::vector<fk::ChunkDev>& sorted = ctx->tmp_chunks2;
+  sorted.resize(chunks.size());
+  std::vector<int> at(first.begin(), first.end() - 1);
+  for (const fk::ChunkDev& c : chunks) sorted[at[cls[c.item]]++] = c;
+  chunks.swap(sorted);
+}
+
+// Lanes per path of an FP64 launch of constant coefficients: 1 (a lane per
+// path, paths_kernel) or 8 or 32 (paths_group_kernel).  Estimated in cycles of
+// an SM: the path-steps at kLaneCost a warp-step, plus the chain of the longest
+// path, which a lane runs step by step after the machine has emptied; with g
+// lanes per path g / 2 steps more per path and a chain g times shorter.  Steps
+// are the mean exit time of the item's start point over h (exact in a disk, a
+// bound from the nearer pair of sides in a rectangle); the longest of n paths
+// is ln(n) decay times of the slowest mode.
+int group_width(const fk_ctx* ctx, const std::vector<fk::ItemDev>& it) {
+  constexpr double kLaneCost = 360, kLaneStep = 2800, kGroupCost = 420, kGroupStep = 3300;
+  double paths = 0, steps = 0, longest = 0;
+  for (const fk::ItemDev& x : it) {
+    if (x.frontera || x.paths == 0) continue;
+    double t = 1e300, decay = 1e300;
+    auto shape = [&](bool circle, const double* p) {
+      if (circle) {  // (r, cx, cy)
+        const double r2 = p[0] * p[0], d2 = (x.x - p[1]) * (x.x - p[1]) + (x.y - p[2]) * (x.y - p[2]);
+        t = std::min(t, 0.25 * std::max(0.0, r2 - d2));
+        decay = std::min(decay, r2 / 5.783);
+      } else {
+        const double w = p[2] - p[0], v = p[3] - p[1];
+        t = std::min(t, 0.5 * std::max(0.0, std::min((x.x - p[0]) * (p[2] - x.x), (x.y - p[1]) * (p[3] - x.y))));
+        decay = std::min(decay, std::min(w * w, v * v) / 9.87);
+      }
+    };
+    const fk::BvpDev& b = ctx->bvps[x.bvp];
+    shape(b.dom_shape == FK_SHAPE_CIRCLE, b.dom);
+    if (x.sub_shape >= 0) shape(x.sub_shape == FK_SHAPE_CIRCLE, x.sub);
+    paths += x.paths;
+    steps += x.paths * (1.0 + t / x.h);
+    longest = std::max(longest, decay / x.h);
+  }
+  longest *= std::log(std::max(2.0, paths));
+  const double warps = 32.0 * ctx->num_sms;
+  int best = 1;
+  double cost = steps / warps * kLaneCost + longest * kLaneStep;
+  for (int g : {8, 32}) {
+    const double c = (steps + 0.5 * g * paths) / warps * kGroupCost + longest / g * kGroupStep;
+    if (c < cost) {
+      cost = c;
+      best = g;
+    }
+  }
+  return best;
+}
+
 int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& it, fk::StencilSet* S,
               const std::vector<long long>* g_off, long long g_total, const int* d_csr_idx, double* d_csr_val,
               const int* d_row, double* d_B, RunOut& out, const RunOpts& o = RunOpts()) {
@@ -561,8 +647,9 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // mode: every warp takes its own chunks and adds the stencil moments to
   // global memory, so an item's slowest path holds up one warp only.  A
   // launch shape set by the caller (fk_set_launch, the autotuner) keeps the
-  // shared chunk slots.
-  bool warp_mode = ctx->chunk <= 0 && n_live > 0 && total_paths <= kWarpModeMaxPaths * n_live;
+  // shared chunk slots, but for FP64 point solves, which have no stencil
+  // moments to share and always run in warp mode.
+  bool warp_mode = (kind == 0 && precision == FK_FP64) || (ctx->chunk <= 0 && n_live > 0 && total_paths <= kWarpModeMaxPaths * n_live);
   // Adaptive rounds with items of few paths: warp mode with per-warp FP32
   // moment accumulators in shared memory, so that the kernel forms the G rows
   // (the rounds keep no moments in global memory).  CTAs of 4 warps (2 for
@@ -583,16 +670,63 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   if (round && warp_mode && !wms) warp_mode = false;  // (rounds need rows formed in the kernel)
   const size_t sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
   if (sacc_bytes > 200 * 1024) return fail(ctx, FK_ERR_CAPACITY, "stencil accumulators exceed shared memory");
-  const int occ = fk::paths_kernel_occupancy(bvp.problem, precision, kind, any_cv ? 1 : 0, lblock, sacc_bytes, warp_mode);
-  const int grid = std::max(1, ctx->num_sms * occ);
-  const int block_used = lblock;
+  int occ = fk::paths_kernel_occupancy(bvp.problem, precision, kind, any_cv ? 1 : 0, lblock, sacc_bytes, warp_mode);
+  // (the 3 CTAs per SM that FP32 slot builds are sized for, also where one needs fewer registers)
+  if (kind == 0 && precision == FK_FP32 && !warp_mode && lblock == 256) occ = std::min(occ, 3);
+  int grid = std::max(1, ctx->num_sms * occ);
+  int block_used = lblock;
+  size_t smem_used = sacc_bytes;
+  int group = 1;  // lanes per path
+  if (warp_mode && ctx->chunk <= 0 && bvp.cv != FK_CV_MLP && fk::paths_group_available(bvp.problem, precision, kind))
+    group = group_width(ctx, it);
+  const bool mix = warp_mode && group == 1 && precision == FK_FP64;
+  if (group > 1) {
+    // as many warps per SM as there are paths for, up to 16 (two CTAs)
+    const long long want = (total_paths * group + 32LL * ctx->num_sms - 1) / (32LL * ctx->num_sms);
+    block_used = static_cast<int>(32 * std::max<long long>(1, std::min<long long>(8, want)));
+    grid = ctx->num_sms * (want > 8 ? 2 : 1);
+  } else if (mix && ctx->chunk <= 0 && block == 256) {
+    // Streaming: full occupancy from 4 paths per lane on; with fewer paths
+    // fewer warps, whose lanes stay busy longer, but one per scheduler at
+    // least (37 anisotropic points x 1,501 paths: 4.0 ms on 4 warps per SM, 4.7
+    // on 16).
+    const int full = occ * lblock / 32;
+    const long long lanes = 32LL * ctx->num_sms;
+    const int wps = static_cast<int>(std::min<long long>(full, std::max<long long>(4, total_paths / (4 * lanes))));
+    if (wps < full) {
+      block_used = wps >= 8 ? 256 : 128;
+      grid = ctx->num_sms * std::max(1, wps * 32 / block_used);
+      // (fewer warps' worth of paths than two per SM: no more warps than that)
+      const long long want = (total_paths + 31) / 32;
+      if (want <= 2LL * ctx->num_sms) {
+        block_used = want <= ctx->num_sms ? 32 : 64;
+        grid = ctx->num_sms;
+      }
+    }
+    smem_used = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, block_used, wms);
+  }
   // Chunk size.  Slots: at least 4 chunks per CTA of the persistent grid, at
   // most 32768 paths.  Warp mode: about 2 chunks per warp, 64..4096 paths
   // (measured on the 8x8 assembly and on point solves, finer chunks cost
   // more in per-chunk work than they save in the last round).  An item is
   // split into equal chunks (no small remainder).
   long long chunk = ctx->chunk;
-  if (chunk <= 0 && warp_mode) {
+  if (group > 1) {
+    // short chunks: a warp takes its chunk's paths 32 / group at a time.  Arc
+    // items of up to 32 paths stay whole: their moments are then summed in one
+    // order, and the ill-conditioned inverse gives the same row in every run.
+    const long long ng = 32 / group;
+    chunk = total_paths / (2LL * grid * (block_used / 32));
+    chunk = std::max<long long>(std::max<long long>(kind == 1 ? 32 : ng, total_paths >> 20), std::min(chunk, 32 * ng));
+  } else if (mix && chunk <= 0) {
+    // Streaming: 64 to 512 paths, about 32 chunks per warp for point solves
+    // (1,024 points x 10^4 paths: 14.9 ms at 64 paths, 15.0 at 128, 16.7 at
+    // 512; but the host lists every chunk, 8 ms for 88 M paths in pieces of
+    // 128) and 8 with a stencil (8x8 FP64 assembly: 15.6 ms at 512,
+    // 15.9 at 128); never more than 2^20 chunks.
+    chunk = total_paths / ((kind == 0 ? 32LL : 8LL) * grid * (block_used / 32));
+    chunk = std::max<long long>(std::max<long long>(64, total_paths >> 20), std::min<long long>(chunk, 512));
+  } else if (chunk <= 0 && warp_mode) {
     chunk = total_paths / (2LL * grid * (block_used / 32));
     chunk = std::max<long long>(64, std::min<long long>(chunk, 4096));
   } else if (chunk <= 0) {
@@ -634,6 +768,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
                        [](const fk::ChunkDev& a, const fk::ChunkDev& b) { return (a.p1 - a.p0) > (b.p1 - b.p0); });
     }
   }
+  std::vector<int>& first = ctx->tmp_first;
+  first.clear();
+  if (mix) group_chunks(ctx, it, chunks, kind, first);
+  const int n_cls = std::max(1, static_cast<int>(first.size()) - 1);
   FK_CUDA(fk::upload_pinned(ctx->w_items, ctx->h_items, it, s));
   FK_CUDA(fk::upload_pinned(ctx->w_chunks, ctx->h_chunks, chunks, s));
   FK_CUDA(ctx->w_stats.ensure(std::max<size_t>(static_cast<size_t>(n) * fk::kNumStats * sizeof(double), 16)));
@@ -668,10 +806,16 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // (until this launch has finished without error, nothing is known to be zero)
   const size_t acc_clean_after = wfuse ? ctx->acc_clean : 0;
   if (!(round || wms)) ctx->acc_clean = 0;
-  FK_CUDA(ctx->w_queue.ensure(32));
   // queue, error word, result flags, windows formed into rows, the first item
   // whose completed path count differs and that count
+  FK_CUDA(ctx->w_queue.ensure(32));
   FK_CUDA(cudaMemsetAsync(ctx->w_queue.p, 0, 7 * sizeof(int), s));
+  if (n_cls > 1) {  // the classes' bounds, then their counters
+    const size_t m = first.size();
+    first.resize(2 * m - 1);
+    std::copy(first.begin(), first.begin() + (m - 1), first.begin() + m);
+    FK_CUDA(fk::upload_pinned(ctx->w_first, ctx->h_first, first, s));
+  }
 
   fk::LaunchArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -708,6 +852,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     a.cv_tex = M.d_tex;
   }
   a.stencil_kind = kind;
+  a.mix = mix ? 1 : 0;
+  a.n_cls = n_cls;
+  a.cls_first = ctx->w_first.as<int>();
+  a.cls_queue = ctx->w_first.as<int>() + n_cls + 1;
   a.acc_words = acc_words;
   a.smem_nodes = smem_nodes;
   // per-item G buffers
@@ -734,8 +882,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     a.g_sum = o.g_sum;
   }
   FK_CUDA(cudaEventRecord(ctx->ev[0], s));
-  if (!chunks.empty())
-    FK_CUDA(fk::launch_paths(a, bvp.problem, precision, grid, block_used, sacc_bytes, s, warp_mode));
+  if (!chunks.empty()) {
+    if (group > 1) FK_CUDA(fk::launch_paths_group(a, bvp.problem, group, grid, block_used, s));
+    else FK_CUDA(fk::launch_paths(a, bvp.problem, precision, grid, block_used, smem_used, s, warp_mode));
+  }
   FK_CUDA(cudaEventRecord(ctx->ev[1], s));
   if (round) {
     FK_CUDA(fk::launch_round_stats(a.items, n, a.stats, o.run_stats, o.item_var, ctx->w_queue.as<int>() + 2, s));

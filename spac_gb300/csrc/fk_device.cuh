@@ -55,14 +55,14 @@ __device__ __forceinline__ uint4 philox10_rk(uint4 c, const uint32_t* rk) {
 // FP64 stepping forms it on the integer pipes (fx::normal_pair, about 230
 // issue slots): the FP64 log, square root and sincos were about 70 of a
 // step's 225 FP64 instructions, 64 slots each.
-__device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, double& z0, double& z1) {
-  fx::normal_pair(a, b, z0, z1);
+__device__ __forceinline__ void box_muller(const fx::Tables* tb, uint32_t a, uint32_t b, double& z0, double& z1) {
+  fx::normal_pair(tb, a, b, z0, z1);
 }
 // FP32 stepping uses the SFU forms (ex2/lg2.approx, sqrt.approx and an
 // approximate division): relative errors ~1e-6 at most, far below the Monte
 // Carlo error of any node estimate.  FP64 stepping keeps the correctly
 // rounded forms (it follows the oracle's paths).
-__device__ __forceinline__ float fexp(float v) { return __expf(v); }
+__device__ __forceinline__ float fexp(const fx::Tables*, float v) { return __expf(v); }
 // 2^v (ex2.approx: the SFU's base-2 exponential)
 __device__ __forceinline__ float fexp2(float v) {
   float r;
@@ -72,8 +72,8 @@ __device__ __forceinline__ float fexp2(float v) {
 // e^v: integer pipes for |v| < 256 (fx::exp_core), which holds every exponent of the
 // registered problems near their domains and every stencil weight that is added
 static __device__ __noinline__ double fexp_far(double v) { return exp(v); }
-__device__ __forceinline__ double fexp(double v) {
-  return (static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu) < 0x40700000u ? fx::exp_core(v) : fexp_far(v);
+__device__ __forceinline__ double fexp(const fx::Tables* tb, double v) {
+  return (static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu) < 0x40700000u ? fx::exp_core(tb, v) : fexp_far(v);
 }
 __device__ __forceinline__ float fsqrt(float v) {
   float r;
@@ -84,7 +84,7 @@ __device__ __forceinline__ double fsqrt(double v) { return sqrt(v); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 
-__device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, float& z0, float& z1) {
+__device__ __forceinline__ void box_muller(const fx::Tables*, uint32_t a, uint32_t b, float& z0, float& z1) {
   const float inv32 = 2.3283064365386962890625e-10f;
   const float u1 = (static_cast<float>(a) + 0.5f) * inv32;  // rounds into (0, 1]
   const float u2 = (static_cast<float>(b) + 0.5f) * inv32;
@@ -222,6 +222,9 @@ struct BvpDev {
   int problem, cv, dom_shape, mlp;
   double dom[4];
   double prob[4];
+  // FP64 stepping's tables, set by each kernel in its copy of the record (shared or global memory)
+  const fx::Tables* tab;
+  float p32[4];  // FP32 stepping of FK_PROBLEM_DISK: prob[0..2] and 1 / (2 prob[2]), likewise
 };
 
 template <typename R>
@@ -255,10 +258,10 @@ struct FrankeEval {
       e3 = fexp2(-0.25f * L2E * s3);
       e4 = fexp2(-L2E * s4);
     } else {
-      e1 = fexp(R(-0.25) * s1);
-      e2 = fexp(R(-1.0 / 49.0) * (c * c) - R(0.1) * d);
-      e3 = fexp(R(-0.25) * s3);
-      e4 = fexp(R(-1) * s4);
+      e1 = fexp(fx::tables(), R(-0.25) * s1);
+      e2 = fexp(fx::tables(), R(-1.0 / 49.0) * (c * c) - R(0.1) * d);
+      e3 = fexp(fx::tables(), R(-0.25) * s3);
+      e4 = fexp(fx::tables(), R(-1) * s4);
     }
   }
   // uxx + uyy with each exponential's two second derivatives combined:
@@ -288,53 +291,54 @@ struct FrankeEval {
 
 // FP64 stepping: the Franke function in fixed point where fx::to_pos holds
 // (the unit square and its surroundings), the FP64 forms elsewhere.
-static __device__ __noinline__ void franke_far(double x, double y, bool grad, double& u, double& lap, double& ux, double& uy) {
+// (Results by value: a variable whose address went to the call would live in
+// local memory on the common path too.)
+struct FrankeFar {
+  double u, lap, ux, uy;
+};
+static __device__ __noinline__ FrankeFar franke_far(double x, double y) {
   const FrankeEval<double> F(x, y);
-  u = F.u();
-  lap = F.lap();
-  if (grad) {
-    ux = F.ux();
-    uy = F.uy();
-  }
+  return FrankeFar{F.u(), F.lap(), F.ux(), F.uy()};
 }
+// (The fixed-point forms run whatever the position, and a position outside
+// their range then overwrites them: without a branch in between, the compiler
+// interleaves them with the step's other work.)
 // Laplacian, and the gradient if asked for.
-__device__ __forceinline__ void franke_lap_grad(double x, double y, bool grad, double& lap, double& ux, double& uy) {
+__device__ __forceinline__ void franke_lap_grad(const fx::Tables* tb, double x, double y, bool grad, double& lap, double& ux, double& uy) {
   fx::i64 X, Y;
   const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
-  if (!ok) {
-    double u;
-    franke_far(x, y, grad, u, lap, ux, uy);
-    return;
-  }
   fx::FrankeArgs f;
   fx::franke_args(X, Y, f);
   if (grad) {
     fx::FrankeTerms b;
     fx::i64 gx, gy;
-    fx::franke_terms(f, b);
+    fx::franke_terms(tb, f, b);
     fx::franke_grad(f, b, gx, gy);
     ux = fx::to_double(gx, -58);
     uy = fx::to_double(gy, -58);
     lap = fx::to_double(fx::franke_lap_terms(f, b), -54);
   } else {
-    lap = fx::to_double(fx::franke_lap(f), -54);
+    lap = fx::to_double(fx::franke_lap(tb, f), -54);
+  }
+  if (__builtin_expect(!ok, 0)) {
+    const FrankeFar F = franke_far(x, y);
+    lap = F.lap;
+    ux = F.ux;
+    uy = F.uy;
   }
 }
-__device__ __forceinline__ double franke_value(double x, double y) {
+__device__ __forceinline__ double franke_value(const fx::Tables* tb, double x, double y) {
   fx::i64 X, Y;
   const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
-  if (!ok) {
-    double u, lap, ux, uy;
-    franke_far(x, y, false, u, lap, ux, uy);
-    return u;
-  }
   fx::FrankeArgs f;
   fx::FrankeTerms b;
   fx::franke_args(X, Y, f);
-  fx::franke_terms(f, b);
-  return fx::to_double(fx::franke_u(b), -60);
+  fx::franke_terms(tb, f, b);
+  double u = fx::to_double(fx::franke_u(b), -60);
+  if (__builtin_expect(!ok, 0)) u = franke_far(x, y).u;
+  return u;
 }
-__device__ __forceinline__ float franke_value(float x, float y) { return FrankeEval<float>(x, y).u(); }
+__device__ __forceinline__ float franke_value(const fx::Tables*, float x, float y) { return FrankeEval<float>(x, y).u(); }
 
 // sin(pi v): SFU form for FP32 stepping (|v| <= 2 here), accurate for FP64
 __device__ __forceinline__ float sinpi_(float v) { return __sinf(3.14159265358979323846f * v); }
@@ -385,14 +389,14 @@ struct Problem<0> {
   template <typename R>
   __device__ static R sigma_of(R) { return R(1.41421356237); }
   template <typename R>
-  __device__ static void step(const BvpDev&, R x, R y, R, R, bool cv, StepCoef<R>& o) {
+  __device__ static void step(const BvpDev& bvp, R x, R y, R, R, bool cv, StepCoef<R>& o) {
     o.s = R(1.41421356237);
     o.c = R(0);
     o.bx = R(0);
     o.by = R(0);
     if constexpr (std::is_same<R, double>::value) {
       double lap, ux, uy;
-      franke_lap_grad(x, y, cv, lap, ux, uy);
+      franke_lap_grad(bvp.tab, x, y, cv, lap, ux, uy);
       o.f = -lap;
       if (cv) {
         o.Fx = -o.s * ux;
@@ -408,12 +412,13 @@ struct Problem<0> {
     }
   }
   template <typename R>
-  __device__ static R u(const BvpDev&, R x, R y) { return franke_value(x, y); }
+  __device__ static R u(const BvpDev& b, R x, R y) { return franke_value(b.tab, x, y); }
 };
 
 // FK_PROBLEM_MONEGROS: sigma = 1.41421356237 I, b = 0, c = -1, f = -Lap u + u.
 template <>
 struct Problem<1> {
+  static constexpr double potential = -1.0;  // c (TraitsOf: constant sigma, no drift, a potential)
   template <typename R>
   __device__ static R state(const BvpDev&, R, R) { return R(0); }
   template <typename R>
@@ -443,11 +448,13 @@ struct Problem<2> {
     return R(1) + R(0.5) * sinpi_(R(2) * x) * sinpi_(R(2) * y);
   }
   template <typename R>
-  __device__ static R state(const BvpDev&, R x, R y) {
+  __device__ static R state(const BvpDev& b, R x, R y) {
     if constexpr (std::is_same<R, double>::value) {
       fx::i64 X, Y;
-      if (fx::to_pos(x, X) & fx::to_pos(y, Y)) return fx::to_double(fx::aniso_a(X, Y), 0u, -62);
-      return a_far(x, y);
+      const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
+      double v = fx::to_double(fx::aniso_a(b.tab, X, Y), 0u, -62);
+      if (__builtin_expect(!ok, 0)) v = a_far(x, y);
+      return v;
     } else {
       return coef_a(x, y);
     }
@@ -477,19 +484,18 @@ struct Problem<2> {
       o.Fy = -o.s * uy;
     }
   }
-  __device__ __noinline__ static void step_far(double x, double y, double a, double s, bool cv, StepCoef<double>& o) {
-    step_of<double>(x, y, a, s, cv, o);
+  __device__ __noinline__ static StepCoef<double> step_far(double x, double y, double a, double s) {
+    StepCoef<double> o;
+    step_of<double>(x, y, a, s, true, o);
+    return o;
   }
   template <typename R>
-  __device__ static void step(const BvpDev&, R x, R y, R a, R s, bool cv, StepCoef<R>& o) {
+  __device__ static void step(const BvpDev& b, R x, R y, R a, R s, bool cv, StepCoef<R>& o) {
     if constexpr (std::is_same<R, double>::value) {
       fx::i64 X, Y;
-      if (!(fx::to_pos(x, X) & fx::to_pos(y, Y))) {
-        step_far(x, y, a, s, cv, o);
-        return;
-      }
+      const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
       fx::AnisoOut p;
-      fx::aniso_step(X, Y, fx::a_bits(a), p);
+      fx::aniso_step(b.tab, X, Y, fx::a_bits(a), p);
       o.s = s;
       o.c = -fx::to_double(p.mc, 0u, -54);
       o.bx = y - 0.5;
@@ -501,12 +507,13 @@ struct Problem<2> {
         o.Fx = -s * fx::to_double(ux, -54);
         o.Fy = -s * fx::to_double(uy, -54);
       }
+      if (__builtin_expect(!ok, 0)) o = step_far(x, y, a, s);
     } else {
       step_of<R>(x, y, a, s, cv, o);
     }
   }
   template <typename R>
-  __device__ static R u(const BvpDev&, R x, R y) { return franke_value(x, y) * (R(1) + x * y); }
+  __device__ static R u(const BvpDev& b, R x, R y) { return franke_value(b.tab, x, y) * (R(1) + x * y); }
 };
 
 // FK_PROBLEM_DISK: Franke mapped from the disk's bounding box to [0,1]^2.
@@ -518,33 +525,42 @@ struct Problem<3> {
   __device__ static R sigma_of(R) { return R(1.41421356237); }
   template <typename R>
   __device__ static void step(const BvpDev& b, R x, R y, R, R, bool cv, StepCoef<R>& o) {
-    const R inv = R(1) / (R(2) * R(b.prob[2]));
-    const R xi = (x - R(b.prob[0])) * inv + R(0.5), eta = (y - R(b.prob[1])) * inv + R(0.5);
-    o.s = R(1.41421356237);
-    o.c = R(0);
-    o.bx = R(0);
-    o.by = R(0);
     if constexpr (std::is_same<R, double>::value) {
+      const R inv = R(1) / (R(2) * R(b.prob[2]));
+      const R xi = (x - R(b.prob[0])) * inv + R(0.5), eta = (y - R(b.prob[1])) * inv + R(0.5);
       double lap, ux, uy;
-      franke_lap_grad(xi, eta, cv, lap, ux, uy);
+      franke_lap_grad(b.tab, xi, eta, cv, lap, ux, uy);
+      o.s = R(1.41421356237);
       o.f = -lap * (inv * inv);
       if (cv) {
         o.Fx = -o.s * ux * inv;
         o.Fy = -o.s * uy * inv;
       }
     } else {
+      // The parameters come converted and inverted once per chunk (read from
+      // the record, each step converted three on the FP64 pipe, 61 % of it, and
+      // divided).  The empty asm hides that they do not change: with loop
+      // constants the compiler fuses other multiplications and additions, and
+      // paths round differently.
+      R p0 = b.p32[0], p1 = b.p32[1], inv = b.p32[3];
+      asm volatile("" : "+f"(p0), "+f"(p1), "+f"(inv));
+      const R xi = (x - p0) * inv + R(0.5), eta = (y - p1) * inv + R(0.5);
       FrankeEval<R> F(xi, eta);
+      o.s = R(1.41421356237);
       o.f = -F.lap() * (inv * inv);
       if (cv) {
         o.Fx = -o.s * F.ux() * inv;
         o.Fy = -o.s * F.uy() * inv;
       }
     }
+    o.c = R(0);
+    o.bx = R(0);
+    o.by = R(0);
   }
   template <typename R>
   __device__ static R u(const BvpDev& b, R x, R y) {
     const R inv = R(1) / (R(2) * R(b.prob[2]));
-    return franke_value((x - R(b.prob[0])) * inv + R(0.5), (y - R(b.prob[1])) * inv + R(0.5));
+    return franke_value(b.tab, (x - R(b.prob[0])) * inv + R(0.5), (y - R(b.prob[1])) * inv + R(0.5));
   }
 };
 
@@ -604,7 +620,8 @@ struct RobinOf<4> {
 };
 
 // What FP64 stepping need not compute for a problem: constant sigma, no drift
-// and no potential (then Y stays 1).
+// and no potential (then Y stays 1).  With the first two, `potential` is the
+// problem's constant c (paths_group_kernel forms a path's steps in parallel).
 template <int PROB>
 struct TraitsOf {
   static constexpr bool const_sigma = PROB != 2 && PROB != 4;

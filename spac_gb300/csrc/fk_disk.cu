@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(kCoefThreads) disk_coef_kernel(const DiskArgs 
   __shared__ int s_var[kCoefThreads / 32];
   const int d = blockIdx.x;
   const DiskDev D = a.disks[d];
-  const BvpDev bvp = *a.bvp;
+  BvpDev bvp = *a.bvp;
+  bvp.tab = fx::tables();
   const int nc = D.nc, n = nc * D.half;
   const double* r = a.tab + D.tab_off + tab_r(D.half);
   double* cg = a.grid + D.grid_off;

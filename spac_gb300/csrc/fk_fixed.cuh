@@ -89,18 +89,19 @@ FX_FN int clz64(u64 v) {
 }
 
 // ------------------------------------------------------------- tables ------
-constexpr u64 kLn2_63 = 0x58B90BFBE8E7BCD6ull;  // ln 2 * 2^63
+constexpr u64 kLn2_64 = 0xB17217F7D1CF79ACull;  // ln 2 * 2^64
 constexpr u64 kLn2_59 = 0x058B90BFBE8E7BCDull;  // ln 2 * 2^59
 
-struct LogEntry {
+struct alignas(16) LogEntry {
   u64 ln;   // -ln(c / 2^16) * 2^59
   u64 c;    // reciprocal of the interval's middle, 16 bits
 };
-struct SinCosEntry {
+struct alignas(16) SinCosEntry {
   u64 c, s;  // cos, sin of the cell's middle * 2^63
 };
-struct Tables {
+struct alignas(16) Tables {
   u64 exp2[1024];       // 2^(j/1024) * 2^62
+  u64 exp2m1[1024];     // (2^(i / 2^20) - 1) * 2^64
   SinCosEntry sc[1024]; // angle (j + 1/2) / 4096 of a turn
   LogEntry log[512];    // y in [1 + j/512, 1 + (j+1)/512)
 };
@@ -125,6 +126,9 @@ constexpr Tables make_tables() {
         v = (p << 1) | 1u;                 // (middle of the dropped bit)
       }
     t.exp2[j] = v >> 1;
+    const u64 x = static_cast<u64>(j) * (kLn2_64 >> 20) + ((static_cast<u64>(j) * (kLn2_64 & 0xfffffu)) >> 20);
+    const u64 x2 = cmulhi(x, x), x3 = cmulhi(x2, x), x4 = cmulhi(x3, x);
+    t.exp2m1[j] = x + x2 / 2 + x3 / 6 + x4 / 24;
   }
   // cos and sin of 2^-i of a turn * 2^64, i = 3 .. 13, then angle (2j + 1) / 8192 from its binary digits
   constexpr u64 cr[11] = {0xB504F333F9DE6484ull, 0xEC835E79946A3145ull, 0xFB14BE7FBAE58156ull, 0xFEC46D1E89292CF0ull,
@@ -178,17 +182,21 @@ constexpr Tables make_tables() {
   }
   return t;
 }
+// The tables in global memory (device) or static storage (host).  The path
+// kernel's warp mode copies them to shared memory: a gather of 32 lanes over
+// 64 cache lines costs a warp that runs alone about 130 cycles there, and ten
+// of them made up 40 % of its step.
 #ifdef __CUDACC__
 static __device__ const Tables kTablesDev = make_tables();
 #endif
 #ifndef __CUDA_ARCH__
 static constexpr Tables kTablesHost = make_tables();
 #endif
-FX_FN const Tables& tables() {
+FX_FN const Tables* tables() {
 #ifdef __CUDA_ARCH__
-  return kTablesDev;
+  return &kTablesDev;
 #else
-  return kTablesHost;
+  return &kTablesHost;
 #endif
 }
 
@@ -224,43 +232,53 @@ FX_FN double to_double(i64 v, int e2) {
   return to_double(static_cast<u64>((v ^ s) - s), static_cast<u32>(s) & 1u, e2);
 }
 
-// -------------------------------------------------------------- exp2 -------
-// 2^(f / 2^54) for the fraction f in [0, 2^54), times 2^62; relative error
-// below 2^-58 (the table's, the truncated products' and the dropped z^5 term).
-FX_FN u64 exp2_frac(u64 f) {
-  const u32 j = static_cast<u32>(f >> 44);
-  // z = (f mod 2^44) 2^-54 ln 2 < 6.8e-4, as z 2^64; e^z - 1 by its series
-  const u64 z = mulhi((f & ((1ull << 44) - 1)) << 11, kLn2_63);
-  const u32 zh = static_cast<u32>(z >> 22), zl = static_cast<u32>(z) & 0x3fffffu;
-  const u64 z2 = ((static_cast<u64>(zh) * zh) >> 21) + ((static_cast<u64>(zh) * zl) >> 42);  // z^2 / 2
-  const u32 z3 = mulhi32(mulhi32(static_cast<u32>(z2 >> 10), 0x55555556u), zh);              // z^3 / 6
-  const u32 z4 = mulhi32(z3, zh) >> 12;                                                      // z^4 / 24
-#ifdef __CUDA_ARCH__
-  const u64 T = __ldg(reinterpret_cast<const unsigned long long*>(&kTablesDev.exp2[j]));
-#else
-  const u64 T = tables().exp2[j];
-#endif
-  return T + mulhi(T, z + z2 + (z3 + z4));
+// -------------------------------------------------------------- exp --------
+// 2^(N / 2^20) e^z for the low 20 bits of N and z 2^64 < 2^45, times 2^62;
+// relative error below 2^-59.  Two tables of ten bits each, so that e^z needs
+// two terms.
+FX_FN u64 exp_frac(const Tables* tb, u32 N, u64 z) {
+  const u32 j = (N >> 10) & 1023u, i = N & 1023u;
+  const u64 T = tb->exp2[j], S = tb->exp2m1[i];
+  const u32 zh = static_cast<u32>(z >> 13);       // z 2^51
+  const u64 w = z + (mulhi32(zh, zh) >> 7);       // e^z - 1 = z + z^2 / 2
+  return T + mulhi(T, S + w + ((static_cast<u64>(static_cast<u32>(S >> 22)) * static_cast<u32>(w >> 13)) >> 29));
 }
-// 2^(q 2^-54) 2^F for q >= -2^62 and a result below 2^63 (truncated).
-template <int F>
-FX_FN u64 exp2_fx(i64 q) {
-  const int sh = 62 - F - static_cast<int>(q >> 54);
-  return exp2_frac(static_cast<u64>(q) & ((1ull << 54) - 1)) >> (sh < 63 ? sh : 63);
+// e^-v for v = V 2^-U >= 0 (V < 2^63, U = 55 or 57): the value is M 2^-62 2^-q, M in [2^62, 2^63 (1 + 2^-19)).
+// n ln 2 / 2^20 lies above v by less than two of its steps; the rest z > 0.
+template <int U>
+FX_FN u64 exp_neg(const Tables* tb, u64 V, int& q) {
+  const u32 n = mulhi32(static_cast<u32>(V >> 32), U == 57 ? 0x0B8AA3B2u : 0x2E2A8ECAu) + 2u;  // log2(e) 2^(84 - U)
+  const u64 z = ((static_cast<u64>(n) * static_cast<u32>(kLn2_64 >> 32)) << 12) +
+                ((static_cast<u64>(n) * static_cast<u32>(kLn2_64)) >> 20) - (V << (64 - U));
+  q = static_cast<int>((n + 0xfffffu) >> 20);
+  return exp_frac(tb, 0u - n, z);
 }
-// e^v for |v| < 256, relative error below 1.1 2^-53 (the rounding of the result and
-// 2^-54 from the exponent's 54 fractional bits).
-FX_FN double exp_core(double v) {
+// e^-v 2^F, truncated (a result below 2^63).
+template <int U, int F>
+FX_FN u64 exp_neg_fx(const Tables* tb, u64 V) {
+  int q;
+  const u64 M = exp_neg<U>(tb, V, q);
+  const int sh = 62 - F + q;
+  return M >> (sh < 63 ? sh : 63);
+}
+// e^v for |v| < 256, relative error below 1.1 2^-53 (the result's rounding).
+FX_FN double exp_core(const Tables* tb, double v) {
   const u64 b = bits_of(v);
   const int e = static_cast<int>(b >> 52) & 0x7ff;
   const u64 m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;  // |v| = m 2^(e - 1085), m < 2^63
-  const int s = 1031 - e;                                                 // > 0 for |v| < 256: |v| 2^54 = m >> s
+  const int s = 1030 - e;                                                 // >= 0 for |v| < 256: |v| 2^55 = m >> s
   const u64 V = s < 63 ? m >> s : 0;
-  // t = |v| log2(e) = V + 0.44 V
-  i64 q = static_cast<i64>(V + mulhi(V, 0x71547652B82FE177ull) + 1);
-  if (b >> 63) q = -q;
-  const u64 M = exp2_frac(static_cast<u64>(q) & ((1ull << 54) - 1));
-  return from_bits((static_cast<u64>(1022 + static_cast<int>(q >> 54)) << 52) + (M >> 10) + ((M >> 9) & 1));
+  const bool neg = (b >> 63) != 0;
+  const u32 n = mulhi32(static_cast<u32>(V >> 32), 0x2E2A8ECAu) + (neg ? 2u : 0u);
+  const u64 nl = ((static_cast<u64>(n) * static_cast<u32>(kLn2_64 >> 32)) << 12) +
+                 ((static_cast<u64>(n) * static_cast<u32>(kLn2_64)) >> 20);
+  const u64 d = nl - (V << 9);
+  const u32 N = neg ? 0u - n : n;
+  u64 M = exp_frac(tb, N, neg ? d : 0ull - d);
+  const int up = static_cast<int>(M >> 63);  // (z may carry the value over the next power of two)
+  M >>= up;
+  const int k = (static_cast<int>(N) >> 20) + up;
+  return from_bits((static_cast<u64>(1022 + k) << 52) + (M >> 10) + ((M >> 9) & 1));
 }
 
 // --------------------------------------------------------- square root -----
@@ -311,17 +329,13 @@ FX_FN u64 sqrt_norm(u64 L, int e, int& e_out) {
 // l = -ln((a + 1/2) 2^-32) as l 2^59 (e = -58) or, in the last table cell
 // before u = 1, l 2^69 (e = -68); absolute error below 2^-55, there 2^-66.
 // Exact argument reduction: u = y 2^(30-n), y c - 1 an integer multiple of 2^-48.
-FX_FN u64 neg_log(u32 a, int& e) {
+FX_FN u64 neg_log(const Tables* tb, u32 a, int& e) {
   const u64 m = (static_cast<u64>(a) << 1) | 1u;
   const int n = clz64(m);
   const u64 Y = m << n;  // y 2^63, y in [1, 2)
   const u32 j = static_cast<u32>(Y >> 54) & 511u;
-#ifdef __CUDA_ARCH__
-  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.log[j]));
-  const u64 ln = t.x, c = t.y;
-#else
-  const u64 ln = tables().log[j].ln, c = tables().log[j].c;
-#endif
+  const LogEntry t = tb->log[j];
+  const u64 ln = t.ln, c = t.c;
   const i64 r = static_cast<i64>((Y >> 31) * c - (1ull << 48));  // (y c - 1) 2^48, |r| < 2^38.1
   const i64 sg = r >> 63;
   const u64 A = static_cast<u64>((r ^ sg) - sg) << 24;  // |r| 2^72
@@ -339,14 +353,10 @@ FX_FN u64 neg_log(u32 a, int& e) {
 
 // cos and sin of the angle b + 1/2 (of 2^32) within its quadrant, times 2^63;
 // absolute error below 2^-58 (the dropped theta^5 / 120 term is 2^-58.6).
-FX_FN void sincos_quadrant(u32 b, u64& cs, u64& sn) {
+FX_FN void sincos_quadrant(const Tables* tb, u32 b, u64& cs, u64& sn) {
   const u32 j = (b >> 20) & 1023u;
-#ifdef __CUDA_ARCH__
-  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.sc[j]));
-  const u64 C = t.x, S = t.y;
-#else
-  const u64 C = tables().sc[j].c, S = tables().sc[j].s;
-#endif
+  const SinCosEntry t = tb->sc[j];
+  const u64 C = t.c, S = t.s;
   // theta = 2 pi D 2^-33 from the cell's middle, |D| < 2^20, odd
   const int D = static_cast<int>(2u * (b & 0xfffffu) + 1u) - (1 << 20);
   const int sg = D >> 31;
@@ -363,17 +373,39 @@ FX_FN void sincos_quadrant(u32 b, u64& cs, u64& sn) {
 }
 
 // Box-Muller pair sqrt(-2 ln u1) (cos, sin)(2 pi u2), u = (word + 1/2) 2^-32:
-// absolute error below 2^-56 for |z| of order 1.
-FX_FN void normal_pair(u32 a, u32 b, double& z0, double& z1) {
-  int el, e;
-  const u64 l = neg_log(a, el);
+// magnitudes m0, m1 times 2^e and signs; absolute error below 2^-56 for |z| of order 1.
+FX_FN void normal_parts(const Tables* tb, u32 a, u32 b, u64& m0, u64& m1, u32& n0, u32& n1, int& e) {
+  int el;
+  const u64 l = neg_log(tb, a, el);
   const u64 rad = sqrt_norm(l, el, e);  // sqrt(2 l) = rad 2^e, rad in [2^60, 2^61]
   u64 c, s;
-  sincos_quadrant(b, c, s);
+  sincos_quadrant(tb, b, c, s);
   const u32 quad = b >> 30;
-  const u64 pc = (quad & 1u) ? s : c, ps = (quad & 1u) ? c : s;
-  z0 = to_double(mulhi(rad, pc), (quad ^ (quad >> 1)) & 1u, e + 1);
-  z1 = to_double(mulhi(rad, ps), quad >> 1, e + 1);
+  m0 = mulhi(rad, (quad & 1u) ? s : c);
+  m1 = mulhi(rad, (quad & 1u) ? c : s);
+  n0 = (quad ^ (quad >> 1)) & 1u;
+  n1 = quad >> 1;
+  e += 1;
+}
+FX_FN void normal_pair(const Tables* tb, u32 a, u32 b, double& z0, double& z1) {
+  u64 m0, m1;
+  u32 n0, n1;
+  int e;
+  normal_parts(tb, a, b, m0, m1, n0, n1, e);
+  z0 = to_double(m0, n0, e);
+  z1 = to_double(m1, n1, e);
+}
+// The pair in 2^-53 units, rounded to nearest (|z| < 6.8, so e <= -57).
+FX_FN void normal_pair_fx(const Tables* tb, u32 a, u32 b, i64& z0, i64& z1) {
+  u64 m0, m1;
+  u32 n0, n1;
+  int e;
+  normal_parts(tb, a, b, m0, m1, n0, n1, e);
+  const int s = -53 - e < 63 ? -53 - e : 63;
+  const u64 half = 1ull << (s - 1);
+  const i64 k0 = -static_cast<i64>(n0), k1 = -static_cast<i64>(n1);
+  z0 = (static_cast<i64>((m0 + half) >> s) ^ k0) - k0;
+  z1 = (static_cast<i64>((m1 + half) >> s) ^ k1) - k1;
 }
 
 // ------------------------------------------------------ Franke function ----
@@ -394,16 +426,14 @@ FX_FN bool to_pos(double v, i64& p) {
   return small && static_cast<u32>(p >> 32) + 0x03000000u < 0x0E000000u;
 }
 constexpr u64 kOne55 = 1ull << 55;
-constexpr u64 kLog2e_4 = 0x5C551D94AE0BF85Eull;  // log2(e) / 4 * 2^64
-
-// Squares (2^-55 units) and base-2 exponents (2^-54) of the four exponentials.
-// One square per coordinate: (9x - k)^2 = (9x)^2 - 2k (9x) + k^2, exact sums.
+// Squares of the four exponents, 2^-55 units.  One square per coordinate:
+// (9x - k)^2 = (9x)^2 - 2k (9x) + k^2, exact sums.
 struct FrankeArgs {
   i64 X9, Y9;       // 9x, 9y (2^-59)
   u64 Gx, Gy;       // (9x)^2, (9y)^2
   u64 s1, s3, s4;   // a^2 + b^2, p^2 + q^2, r^2 + t^2
   u64 c2;           // (9x + 1)^2
-  i64 t1, t2, t3, t4;  // e_i = 2^-t_i
+  i64 v2;           // (9x + 1)^2 / 49 + (9y + 5) / 10 (2^-57): e2 = e^(4/10 - v2)
 };
 FX_FN u64 abs64(i64 v) {
   const i64 s = v >> 63;
@@ -420,19 +450,15 @@ FX_FN void franke_args(i64 X, i64 Y, FrankeArgs& f) {
   f.s3 = static_cast<u64>(S - (f.X9 - xe) - (yq + ye)) + 58 * kOne55;
   f.s4 = static_cast<u64>(S - (f.X9 >> 1) - (f.Y9 - ye)) + 65 * kOne55;
   f.c2 = f.Gx + 2 + static_cast<u64>(xe) + kOne55;
-  f.t1 = static_cast<i64>((mulhi(f.s1, kLog2e_4) + 1) >> 1);
-  f.t3 = static_cast<i64>((mulhi(f.s3, kLog2e_4) + 1) >> 1);
-  f.t4 = static_cast<i64>((f.s4 + mulhi(f.s4, 0x71547652B82FE177ull) + 1) >> 1);
-  // (9x + 1)^2 / 49 + (9y + 5) / 10 - 4 / 10, times log2(e)
-  const u64 d = static_cast<u64>(f.Y9 >> 1) + (5ull << 58);
-  f.t2 = static_cast<i64>((mulhi(f.c2, 0x07898F79D9F68737ull) >> 1) + (mulhi(d, 0x24EED8A1DF37FCF2ull) >> 4) - 0x0024EED8A1DF37FCull);
+  f.v2 = static_cast<i64>(mulhi(f.c2, 0x14E5E0A72F053978ull) + mulhi(static_cast<u64>(f.Y9 >> 1) + (5ull << 58), 0x0CCCCCCCCCCCCCCDull));
 }
-// Laplacian of the Franke function, 2^-54 units; each coefficient is folded
-// into its exponential's exponent (log2 of 243/16, 486/4802, 81/8, 324/5):
+// Laplacian of the Franke function, 2^-54 units; each coefficient c is folded
+// into its exponential's exponent as m ln 2 - ln c >= 0, the power of two into its scale:
 // lap = 243/16 (s1 - 4) e1 + 81/8 (s3 - 4) e3 - 324/5 (s4 - 1) e4 + 486/4802 (c2 - 18.4975) e2
-FX_FN i64 franke_lap(const FrankeArgs& f) {
-  const u64 E1 = exp2_fx<59>(70703136514952234ll - f.t1), E3 = exp2_fx<59>(60165388913858184ll - f.t3);
-  const u64 E4 = exp2_fx<56>(108409243449604861ll - f.t4), E2 = exp2_fx<62>(-59530510741125490ll - f.t2);
+FX_FN i64 franke_lap(const Tables* tb, const FrankeArgs& f) {
+  const u64 E1 = exp_neg_fx<57, 59 + 4>(tb, f.s1 + 0x001AAEF2D0FB10FCull), E3 = exp_neg_fx<57, 59 + 4>(tb, f.s3 + 0x00EA481236F7D35Cull);
+  const u64 E4 = exp_neg_fx<55, 56 + 7>(tb, f.s4 + 0x005721FC55588EF9ull);
+  const u64 E2 = exp_neg_fx<57, 62 - 2>(tb, static_cast<u64>(f.v2) + 0x0102319DC0F73A58ull);
   i64 l = static_cast<i64>(mulshr<60>(f.s1, E1)) - static_cast<i64>(E1 >> 3);
   l += static_cast<i64>(mulshr<60>(f.s3, E3)) - static_cast<i64>(E3 >> 3);
   l -= static_cast<i64>(mulshr<57>(f.s4, E4)) - static_cast<i64>(E4 >> 2);
@@ -443,11 +469,11 @@ FX_FN i64 franke_lap(const FrankeArgs& f) {
 struct FrankeTerms {
   u64 b1, b2, b3, b4;
 };
-FX_FN void franke_terms(const FrankeArgs& f, FrankeTerms& b) {
-  b.b1 = exp2_fx<60>(-7476650908387934ll - f.t1);
-  b.b2 = exp2_fx<60>(-7476650908387934ll - f.t2);
-  b.b3 = exp2_fx<59>(-f.t3);
-  b.b4 = exp2_fx<60>(-41828138011663243ll - f.t4);
+FX_FN void franke_terms(const Tables* tb, const FrankeArgs& f, FrankeTerms& b) {
+  b.b1 = exp_neg_fx<57, 60>(tb, f.s1 + 0x00934B1089A6DC94ull);
+  b.b2 = exp_neg_fx<57, 60 + 1>(tb, static_cast<u64>(f.v2) + 0x01296273AC7DAEBAull);
+  b.b3 = exp_neg_fx<57, 59>(tb, f.s3);
+  b.b4 = exp_neg_fx<55, 60 - 2>(tb, f.s4 + 0x001C8FF7C79A9A22ull);
 }
 FX_FN i64 franke_u(const FrankeTerms& b) { return static_cast<i64>(b.b1 + b.b2 + b.b3 - b.b4); }
 // u_x and u_y, 2^-58 units (g = 18/49):
@@ -475,14 +501,10 @@ FX_FN i64 franke_lap_terms(const FrankeArgs& f, const FrankeTerms& b) {
 
 // -------------------------------------- the anisotropic problem's factors ----
 // sin(2 pi x), 2^-63 units and its sign; x in 2^-59 units of a turn.
-FX_FN u64 sin_turn(i64 X, u32& neg) {
+FX_FN u64 sin_turn(const Tables* tb, i64 X, u32& neg) {
   const u32 quad = static_cast<u32>(X >> 57) & 3u, j = static_cast<u32>(X >> 47) & 1023u;
-#ifdef __CUDA_ARCH__
-  const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(&kTablesDev.sc[j]));
-  const u64 C = t.x, S = t.y;
-#else
-  const u64 C = tables().sc[j].c, S = tables().sc[j].s;
-#endif
+  const SinCosEntry t = tb->sc[j];
+  const u64 C = t.c, S = t.s;
   const i64 D = (X & ((1ll << 47) - 1)) - (1ll << 46);  // theta = 2 pi D 2^-59 from the cell's middle
   const i64 sg = D >> 63;
   const u64 th = mulhi(static_cast<u64>((D ^ sg) - sg) << 17, 0x6487ED5110B4611Aull);  // theta 2^72
@@ -496,9 +518,9 @@ FX_FN u64 sin_turn(i64 X, u32& neg) {
   return P - mulhi(P, c1 << 1) + ((mulhi(Q, s1 << 1) ^ m) - m);
 }
 // a = 1 + sin(2 pi x) sin(2 pi y) / 2, 2^-62 units
-FX_FN u64 aniso_a(i64 X, i64 Y) {
+FX_FN u64 aniso_a(const Tables* tb, i64 X, i64 Y) {
   u32 nx, ny;
-  const u64 sx = sin_turn(X, nx), sy = sin_turn(Y, ny);
+  const u64 sx = sin_turn(tb, X, nx), sy = sin_turn(tb, Y, ny);
   const u64 p = mulhi(sx, sy) >> 1;
   const u64 m = 0ull - static_cast<u64>(nx ^ ny);
   return (1ull << 62) + ((p ^ m) - m);
@@ -522,11 +544,11 @@ struct AnisoOut {
   u64 mc;
   i64 F, Fx, Fy, q;  // 2^-60, 2^-58, 2^-58, 2^-60 units
 };
-FX_FN void aniso_step(i64 X, i64 Y, u64 a62, AnisoOut& o) {
+FX_FN void aniso_step(const Tables* tb, i64 X, i64 Y, u64 a62, AnisoOut& o) {
   FrankeArgs f;
   FrankeTerms b;
   franke_args(X, Y, f);
-  franke_terms(f, b);
+  franke_terms(tb, f, b);
   o.F = franke_u(b);
   franke_grad(f, b, o.Fx, o.Fy);
   const i64 lap = franke_lap_terms(f, b);

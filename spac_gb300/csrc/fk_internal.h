@@ -146,6 +146,12 @@ struct LaunchArgs {
   // G row goes into the CSR values (and item_G if set); 2: adaptive rounds,
   // the chunk's unnormalised row is added to g_sum.
   int fuse_g;
+  // streaming launches: classes of chunks with equal constants (n_cls > 1:
+  // class c is chunks cls_first[c] .. cls_first[c + 1] - 1, with a counter each)
+  int n_cls;
+  const int* cls_first;
+  int* cls_queue;          // n_cls counters, each at its class's first chunk before launch
+  int mix;                 // warp mode: a warp goes on to the next chunk before its lanes have drained (same parameters)
   int wm_shared;           // warp mode: moments in per-warp shared FP32 accumulators, rows fused
   const float* patch_e32;  // FP32 moments: E_W = A_W^-1 - I, the layout of the FP64 inverses
   const double* patch_ainv;  // FP64 moments: A_W^-1
@@ -212,7 +218,12 @@ size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block,
                          size_t smem, cudaStream_t s, bool warp_mode = false);
 // path-kernel builds without the control-variate terms (fk_paths_plain.cu)
-const void* select_paths_plain(int problem, int precision, int st, bool warp_mode, bool four);
+const void* select_paths_plain(int problem, int precision, int st, bool warp_mode, bool alt);
+// time-parallel kernel (fk_paths_group.cu): g lanes (8 or 32) per path, FP64
+// stepping of point solves and arc stencils for problems of constant
+// coefficients, no learned control variate
+bool paths_group_available(int problem, int precision, int stencil_kind);
+cudaError_t launch_paths_group(const LaunchArgs& a, int problem, int g, int grid, int block, cudaStream_t s);
 int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem,
                            bool warp_mode = false);
 // host launchers (fk_kernels.cu)

@@ -26,7 +26,8 @@ constexpr int kFinalizeThreads = 512;
 template <int PROB>
 __device__ __forceinline__ void finalize_item_head(const FinalizeArgs& a, int item, const ItemDev& it, bool live,
                                                    double N) {
-  const BvpDev bvp = a.bvp[it.bvp];
+  BvpDev bvp = a.bvp[it.bvp];
+  bvp.tab = fx::tables();
   const double* S = a.stats + static_cast<long long>(item) * kNumStats;
   double Bv;
   if (it.frontera) {

@@ -8,17 +8,17 @@ namespace fk {
 
 namespace {
 
-const void* select_paths_v(int problem, int precision, int st, bool warp_mode, bool four, bool cv) {
-  if (!cv) return select_paths_plain(problem, precision, st, warp_mode, four);
+const void* select_paths_v(int problem, int precision, int st, bool warp_mode, bool alt, bool cv) {
+  if (!cv) return select_paths_plain(problem, precision, st, warp_mode, alt);
   if (warp_mode)
-    return precision == 1 ? paths_fn_r<float, true, true>(problem, st, false)
-                          : paths_fn_r<double, true, true>(problem, st, false);
-  return precision == 1 ? paths_fn_r<float, false, true>(problem, st, four)
-                        : paths_fn_r<double, false, true>(problem, st, false);
+    return precision == 1 ? paths_fn_r<float, true, true>(problem, st, alt)
+                          : paths_fn_r<double, true, true>(problem, st, alt);
+  return precision == 1 ? paths_fn_r<float, false, true>(problem, st, alt)
+                        : paths_fn_r<double, false, true>(problem, st, alt);
 }
 // The variant a launch uses: the 4-CTA build for FP32 patch-stencil slot
 // mode when 4 of its CTAs fit on an SM with this shared memory and block.
-const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv) {
+const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv, int n_cls) {
   if (precision == 1 && st == 2 && !warp_mode && block == 256) {
     const void* f4 = select_paths_v(problem, precision, st, warp_mode, true, cv);
     int n = 0;
@@ -27,7 +27,7 @@ const void* select_paths(int problem, int precision, int st, bool warp_mode, int
       return f4;
     cudaGetLastError();
   }
-  return select_paths_v(problem, precision, st, warp_mode, false, cv);
+  return select_paths_v(problem, precision, st, warp_mode, st == 0 && n_cls > 1, cv);
 }
 
 }  // namespace
@@ -35,15 +35,15 @@ const void* select_paths(int problem, int precision, int st, bool warp_mode, int
 size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem_nodes, bool warp_mode, int block,
                         bool wm_shared) {
   if (warp_mode)
-    return static_cast<size_t>(block / 32) *
-           paths_slot_bytes(precision, stencil_kind, wm_shared ? acc_words : 0, smem_nodes);
+    return (precision == 0 ? sizeof(fx::Tables) : 0) +
+           static_cast<size_t>(block / 32) * paths_slot_bytes(precision, stencil_kind, wm_shared ? acc_words : 0, smem_nodes);
   return static_cast<size_t>(paths_slots(precision)) * paths_slot_bytes(precision, stencil_kind, acc_words, smem_nodes);
 }
 
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block, size_t smem,
                          cudaStream_t s, bool warp_mode) {
   if (block < 32 || block > 256 || block % 32 != 0) return cudaErrorInvalidValue;
-  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0);
+  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0, a.n_cls);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<LaunchArgs*>(&a)};
@@ -51,7 +51,7 @@ cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int gr
 }
 
 int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem, bool warp_mode) {
-  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0);
+  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0, 1);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess) return 1;

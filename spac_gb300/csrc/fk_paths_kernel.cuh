@@ -91,8 +91,12 @@ struct SAccType {
 // Per-warp queue of exits awaiting processing (exit point, Y, Z, xi, and
 // steps | domain-exit << 30 | capped << 31); at most 31 + 32 entries.
 constexpr int kMaxBlockWarps = 8;
-template <typename R>
-struct ExitQueue {
+struct NoItems {};
+struct ExitItems {
+  int it[64];  // warp mode: the exit's item
+};
+template <typename R, bool MIX>
+struct ExitQueue : std::conditional<MIX, ExitItems, NoItems>::type {
   R x[64], y[64], Y[64], Z[64], xi[64];
   unsigned kf[64];
 };
@@ -109,9 +113,20 @@ struct PatchSh {
   R knn_u0[4];
 };
 
+// Streaming (FP64 warp mode): the warp's class of chunks (its index, end and
+// counter) and the classes it has not been in, kept out of the registers of the
+// step loop.
+template <typename R>
+struct ClassSh {};
+template <>
+struct ClassSh<double> {
+  int cls, cls_hi, cls_left;
+  int* cls_next;
+};
+
 // A chunk slot.  `ready` is written last, after the slot's contents.
 template <typename R>
-struct SlotSh {
+struct SlotSh : ClassSh<R> {
   int ready;        // position in the CTA's chunk sequence that the slot holds
   int chunk;        // chunk index; -1: the chunk queue was exhausted
   int warps_left;   // warps that have not yet left the chunk
@@ -525,6 +540,152 @@ __device__ void fused_patch_row(const LaunchArgs& a, const ItemDev& itg, int ite
   __syncwarp();
 }
 
+// FP64 stepping: the function tables into shared memory (all loads of a
+// thread's part in flight).
+__device__ __forceinline__ void stage_tables(unsigned char* smem) {
+  constexpr int n = static_cast<int>(sizeof(fx::Tables) / 16);
+  const uint4* src = reinterpret_cast<const uint4*>(fx::tables());
+  uint4* dst = reinterpret_cast<uint4*>(smem);
+  for (int i0 = 0; i0 < n; i0 += 10 * blockDim.x) {
+    uint4 v[10];
+#pragma unroll
+    for (int j = 0; j < 10; ++j) {
+      const int i = i0 + j * blockDim.x + threadIdx.x;
+      if (i < n) v[j] = __ldg(src + i);
+    }
+#pragma unroll
+    for (int j = 0; j < 10; ++j) {
+      const int i = i0 + j * blockDim.x + threadIdx.x;
+      if (i < n) dst[i] = v[j];
+    }
+  }
+  __syncthreads();
+}
+
+// A subdomain strictly inside the rectangular domain is always nearer (in
+// Dentro's signed distance) than the domain boundary, wherever the path is,
+// so the domain distance cannot decide an exit and is not evaluated.
+template <int PROB, typename R>
+__device__ __forceinline__ bool domain_can_win(bool has_sub, bool sub_circle, R d0, R d1, R d2, R d3, R s0, R s1, R s2, R s3) {
+  if (has_sub && DomainOf<PROB>::shape == 0) {
+    if (sub_circle)  // (r, cx, cy)
+      return !(s1 - s0 > d0 && s1 + s0 < d2 && s2 - s0 > d1 && s2 + s0 < d3);
+    return !(s0 > d0 && s1 > d1 && s2 < d2 && s3 < d3);  // (x0, y0, x1, y1)
+  }
+  return true;
+}
+
+// Dentro's boundary for a path that stops (FeynmanKacSolver.cpp:68-106): the
+// larger signed distance decides, a tie goes to the domain.
+template <int PROB, typename R>
+__device__ __forceinline__ void dentro_exit(R x, R y, bool dom_can_win, bool has_sub, bool sub_circle, R d0, R d1, R d2, R d3,
+                                            R s0, R s1, R s2, R s3, Bnd<R>& w, bool& dom_wins) {
+  dom_wins = true;
+  if (dom_can_win) {
+    w = (DomainOf<PROB>::shape == 1) ? circle_dist<R>(x, y, d0, d1, d2) : rect_dist<R>(x, y, d0, d1, d2, d3);
+    if (has_sub) {
+      const Bnd<R> sb = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
+      if (!(w.d >= sb.d)) { w = sb; dom_wins = false; }
+    }
+  } else {
+    w = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
+    dom_wins = false;
+  }
+}
+
+// FP64 stepping: the exit test of Dentro with few FP64 instructions (one
+// takes 64 issue slots here).  A path goes on iff every boundary's signed
+// distance is below the (negative) threshold, so the distances alone are
+// formed, from centres and half sides kept here; a circle's test compares
+// squared radii, without the square root.  Dentro's choice of boundary,
+// projection and normal follow only when some lane of the warp stops.
+template <int PROB>
+struct ExitTest {
+  bool dom, sub, circle;
+  double dcx, dcy, dhx, dhy, scx, scy, shx, shy, thr;
+  __device__ __forceinline__ ExitTest(bool dom_can_win, bool has_sub, bool sub_circle, double d0, double d1, double d2, double d3,
+                                      double s0, double s1, double s2, double s3, double thr_)
+      : dom(dom_can_win), sub(has_sub), circle(sub_circle), dcx(d1), dcy(d2), dhx(d0), dhy(0.0), scx(s1), scy(s2), shx(s0),
+        shy(0.0), thr(thr_) {
+    if (DomainOf<PROB>::shape == 0) {
+      dcx = 0.5 * (d0 + d2); dcy = 0.5 * (d1 + d3); dhx = d2 - dcx; dhy = d3 - dcy;
+    }
+    if (!sub_circle) {
+      scx = 0.5 * (s0 + s2); scy = 0.5 * (s1 + s3); shx = s2 - scx; shy = s3 - scy;
+    }
+  }
+  // d < thr < 0 of a rectangle: the larger of two negative offsets, as integers (a
+  // negative double grows as its bits fall; a non-negative or NaN offset fails)
+  __device__ __forceinline__ bool rect_in(double x, double y, double cx, double cy, double hx, double hy) const {
+    const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
+    return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
+  }
+  // |x - c|, at least 5e-4, below r0 + thr
+  __device__ __forceinline__ bool circle_in(double x, double y, double r0, double cx, double cy) const {
+    const double nx = x - cx, ny = y - cy, rho = r0 + thr;
+    return rho > 5e-4 && nx * nx + ny * ny < rho * rho;
+  }
+  __device__ __forceinline__ bool inside(double x, double y) const {
+    bool in = true;
+    if (dom) in = DomainOf<PROB>::shape == 1 ? circle_in(x, y, dhx, dcx, dcy) : rect_in(x, y, dcx, dcy, dhx, dhy);
+    if (sub) in = in && (circle ? circle_in(x, y, shx, scx, scy) : rect_in(x, y, scx, scy, shx, shy));
+    return in;
+  }
+};
+
+struct NoExitTest {
+  template <typename... A>
+  __device__ __forceinline__ explicit NoExitTest(A...) {}
+};
+
+// A warp's thread sums into the item's FP64 sums.
+template <bool CV, typename Acc>
+__device__ __forceinline__ void add_item_sums(const LaunchArgs& a, int item, const Acc* acc, unsigned long long n_steps,
+                                              unsigned n_dom, unsigned n_cap, unsigned n_done, int lane) {
+  double* sums = a.stats + static_cast<long long>(item) * kNumStats;
+  const int slot_of[kNumAcc] = {kStatScore, kStatScore2, kStatXiAlias, kStatVR, kStatVR2, kStatXiScore, kStatB, kStatXi2};
+#pragma unroll
+  for (int j = 0; j < kNumAcc; ++j) {
+    if (!CV && j != 0 && j != 1 && j != 6) continue;
+    const double t = warp_reduce(acc[j], lane);
+    if (lane == 0 && t != 0.0) {
+      atomicAdd(&sums[slot_of[j]], t);
+      if (!CV && j < 2) atomicAdd(&sums[slot_of[j + 3]], t);  // score -> VR, score^2 -> VR^2
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    n_steps += __shfl_xor_sync(kFull, n_steps, o);
+    n_dom += __shfl_xor_sync(kFull, n_dom, o);
+    n_cap += __shfl_xor_sync(kFull, n_cap, o);
+    n_done += __shfl_xor_sync(kFull, n_done, o);
+  }
+  if (lane == 0) {
+    if (n_steps) atomicAdd(&sums[kStatSteps], static_cast<double>(n_steps));
+    if (n_dom) atomicAdd(&sums[kStatDom], static_cast<double>(n_dom));
+    if (n_cap) atomicAdd(&sums[kStatCap], static_cast<double>(n_cap));
+    if (n_done) atomicAdd(&sums[kStatPaths], static_cast<double>(n_done));
+  }
+}
+
+// Interfaz::Update_G moments of the exits in the lanes `im` (angles th,
+// weights Y) into an item's accumulators, lanes over the arc's n <= 64 nodes.
+__device__ __forceinline__ void add_arc_moments(double* acc, unsigned im, double th, double Y, const double* sth, int n,
+                                                double c2, int lane) {
+  double m0 = 0.0, m1 = 0.0;
+  const double t0 = lane < n ? sth[lane] : 0.0, t1 = lane + 32 < n ? sth[lane + 32] : 0.0;
+  while (im) {
+    const int src = __ffs(im) - 1;
+    im &= im - 1;
+    const double tb = __shfl_sync(kFull, th, src), Yb = __shfl_sync(kFull, Y, src);
+    const double d0 = tb - t0, d1 = tb - t1;
+    m0 += Yb / sqrt(d0 * d0 + c2);
+    if (n > 32) m1 += Yb / sqrt(d1 * d1 + c2);
+  }
+  if (lane < n) atomicAdd(&acc[lane], m0);
+  if (lane + 32 < n) atomicAdd(&acc[lane + 32], m1);
+}
+
 // FP64 stepping is bound by the FP64 pipe, not by latency: it trades
 // occupancy for registers (2 CTAs of 256 per SM instead of 3).
 //
@@ -540,15 +701,27 @@ __device__ void fused_patch_row(const LaunchArgs& a, const ItemDev& itg, int ite
 // admits 4 CTAs: it runs the 8x8 assembly 2.9 % faster, while point solves,
 // warp mode and the larger patches of the 32x32 mesh measured slower at 64
 // registers.
-template <typename R, int PROB, int ST, bool WM, int MB, bool CV>
+// CLS: streaming with more than one class of chunks.  Point solves also have a
+// build without: the class bookkeeping, though it runs once per chunk, costs
+// the step loop 12 to 18 % of its latency (one point x 1,000 paths: 0.53
+// against 0.46 ms), and most calls have one class.
+template <typename R, int PROB, int ST, bool WM, int MB, bool CV, bool CLS>
 __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
   using SAcc = typename std::conditional<WM, double, typename SAccType<R, ST>::type>::type;
   using Acc = typename std::conditional<std::is_same<R, double>::value, AccD, AccK>::type;
   constexpr int kPrec = std::is_same<R, double>::value ? 0 : 1;
+  // streaming builds (below): FP64 stepping.  FP32 keeps its chunks apart: its
+  // thread sums round to 2^-24 of a path's score at every addition, so another
+  // partition of the paths moves a mean of a few hundred paths by 4e-9, and its
+  // stencil launches of warp mode form their rows per item in the kernel.
+  constexpr bool kMix = WM && std::is_same<R, double>::value;
+  // FP64 stepping in warp mode: the function tables at the start of the shared memory
+  constexpr bool kShTab = WM && kPrec == 0;
+  constexpr size_t kTab = kShTab ? sizeof(fx::Tables) : 0;
   constexpr int S = WM ? kMaxBlockWarps : (kPrec == 0 ? 2 : kSlotsFP32);  // slots, or one per warp
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SlotSh<R> slots[S];
-  __shared__ ExitQueue<R> sq[kMaxBlockWarps];
+  __shared__ ExitQueue<R, kMix> sq[kMaxBlockWarps];
   // warp mode with per-warp FP32 moment accumulators in shared memory (FP32
   // patch stencils): the warp forms its chunk's G row itself when it leaves
   constexpr bool kWmsCapable = WM && ST == 2 && std::is_same<R, float>::value;
@@ -563,6 +736,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       a.wait_limit_ns ? a.wait_limit_ns : 60000000000ull + 1000ull * static_cast<unsigned long long>(a.max_steps);
   const int n_chunks = a.n_chunks_dev ? *a.n_chunks_dev : a.n_chunks;
 
+  if constexpr (kShTab) stage_tables(smem_raw);
   if (!WM) {
     if (threadIdx.x < S) slots[threadIdx.x].ready = -1;
     __syncthreads();
@@ -570,27 +744,73 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       fill_slot<R, ST>(a, n_chunks, slots[s], smem_raw + s * slot_bytes, acc_bytes, s, nwarps, lane);
   }
 
-  ExitQueue<R>& q = sq[warp];
+  ExitQueue<R, kMix>& q = sq[warp];
   // Slots known to hold no further chunk: a slot whose chunk queue came up
   // empty is never refilled, so the walk ends once every slot is dead.
   unsigned dead = 0u;
+  // Warp mode: the warp's next chunk; with streaming (a.mix) claimed ahead by
+  // lane 0 (`ahead`) and broadcast only when it is needed.  The chunks of a
+  // streaming launch lie in classes of equal constants, each with its own
+  // counter (which starts at the class's first chunk): a warp starts in the
+  // class at its share of the chunk list, stays in it while it lasts and goes
+  // round the others then, so that it drains once per class it visits (one
+  // shared list in class order made every warp drain in every class: 24
+  // against 17 ms on the circle mesh).
+  int ahead = -1, nxt = -1;
+  if constexpr (kMix) {
+    if (lane == 0) {
+      SlotSh<R>& w = slots[warp];
+      w.cls = 0;
+      w.cls_left = 1;
+      w.cls_hi = n_chunks;
+      w.cls_next = a.queue;
+      if (CLS && a.n_cls > 1) {
+        const int nw = gridDim.x * nwarps, me = blockIdx.x + warp * gridDim.x;
+        const int at = static_cast<int>(static_cast<long long>(me) * n_chunks / nw);
+        int k = 0;
+        while (k + 1 < a.n_cls && a.cls_first[k + 1] <= at) ++k;
+        w.cls = k;
+        w.cls_left = a.n_cls;
+        w.cls_hi = a.cls_first[k + 1];
+        w.cls_next = a.cls_queue + k;
+      }
+      if (a.mix) ahead = atomicAdd(CLS ? w.cls_next : a.queue, 1);
+    }
+    __syncwarp();
+  }
   for (int g = 0;; ++g) {
     int si, c;
     if (WM) {
-      // this warp's next chunk
       si = warp;
-      int cc = 0;
-      if (lane == 0) cc = atomicAdd(a.queue, 1);
-      c = __shfl_sync(kFull, cc, 0);
-      if (c >= n_chunks) break;
+      if (!(kMix && a.mix) && lane == 0) ahead = atomicAdd(a.queue, 1);
+      c = kMix && nxt >= 0 ? nxt : __shfl_sync(kFull, ahead, 0);
+      nxt = -1;
+      if constexpr (kMix) {
+        if (lane == 0) {
+          SlotSh<R>& w = slots[warp];
+          while (CLS && c >= w.cls_hi && --w.cls_left > 0) {  // the class has run out: the next one's
+            w.cls = w.cls + 1 < a.n_cls ? w.cls + 1 : 0;
+            w.cls_hi = a.cls_first[w.cls + 1];
+            w.cls_next = a.cls_queue + w.cls;
+            c = atomicAdd(w.cls_next, 1);
+          }
+          if (c >= (CLS ? w.cls_hi : n_chunks)) c = n_chunks;
+          else if (a.mix) ahead = atomicAdd(CLS ? w.cls_next : a.queue, 1);
+        }
+        c = __shfl_sync(kFull, c, 0);
+        __syncwarp();
+        if (c >= n_chunks) break;
+      } else {
+        if (c >= n_chunks) break;
+      }
       if (wms) {
-        uint4* z = reinterpret_cast<uint4*>(smem_raw + si * slot_bytes);
+        uint4* z = reinterpret_cast<uint4*>(smem_raw + kTab + si * slot_bytes);
         for (int i = lane; i < static_cast<int>(acc_bytes / 16); i += 32) z[i] = make_uint4(0u, 0u, 0u, 0u);
       }
-      stage_stencil<R, ST>(a, slots[si], smem_raw + si * slot_bytes + acc_bytes, a.items[a.chunks[c].item].stencil,
+      stage_stencil<R, ST>(a, slots[si], smem_raw + kTab + si * slot_bytes + acc_bytes, a.items[a.chunks[c].item].stencil,
                            lane);
       if (wfuse) {
-        unsigned* vm = reinterpret_cast<unsigned*>(smem_raw + si * slot_bytes + acc_bytes +
+        unsigned* vm = reinterpret_cast<unsigned*>(smem_raw + kTab + si * slot_bytes + acc_bytes +
                                                    paths_slot_nodes_bytes(kPrec, ST, a.smem_nodes));
         for (int i = lane; i < (a.smem_nodes + 31) / 32; i += 32) vm[i] = 0u;
       }
@@ -610,7 +830,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       }
     }
     SlotSh<R>& sl = slots[si];
-    unsigned char* mem = smem_raw + si * slot_bytes;
+    unsigned char* mem = smem_raw + kTab + si * slot_bytes;
     const ChunkDev ch = a.chunks[c];
     const ItemDev& itg = a.items[ch.item];
     // stencil moments: the slot's shared accumulators, or (warp mode) the
@@ -623,49 +843,41 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     const double* sth = reinterpret_cast<const double*>(mem + acc_bytes);
     const PatchSh<R>& sp = sl.sp;
     const ArcDev& sarc = sl.sarc;
-    const unsigned n_ch = ch.p1 - ch.p0;
+    unsigned n_ch = ch.p1 - ch.p0;
+    // Streaming (warp mode, a.mix): once the chunk's paths are all taken, the
+    // lanes that finish go on with the next chunk while the others are still
+    // on their way, provided its item has the same step size, problem,
+    // subdomain and stencil (the warp's constants); the warp drains only where
+    // they differ and at the end of the launch.  cur: the item whose paths are
+    // being started and whose sums the threads hold.
+    int cur = ch.item;
+    unsigned p0 = ch.p0;
+    bool stop = !kMix || !a.mix;  // no chunk may join before the lanes have drained
 
     // the item's BVP (independent problems of one functor share a launch; the
     // control variate is the item's own, so learned-CV items and their plain
     // fallback can share one launch)
-    const BvpDev bvp = a.bvp[itg.bvp];  // (a copy: the problem parameters are converted once per chunk, not per step)
+    BvpDev bvp = a.bvp[itg.bvp];  // (a copy: parameters converted once per chunk)
+    bvp.tab = kShTab ? reinterpret_cast<const fx::Tables*>(smem_raw) : fx::tables();
+    if constexpr (DomainOf<PROB>::shape == 1 && kPrec == 1) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) bvp.p32[i] = static_cast<float>(bvp.prob[i]);
+      bvp.p32[3] = 1.0f / (2.0f * bvp.p32[2]);
+    }
     const bool cv_exact = CV && bvp.cv == 1;                // F from the problem functor
     const bool cv_table = CV && a.cv == 2 && bvp.cv == 2;   // F from the learned gradient table
     const bool cv = cv_exact || cv_table;             // any control term
     const R d0 = R(bvp.dom[0]), d1 = R(bvp.dom[1]), d2 = R(bvp.dom[2]), d3 = R(bvp.dom[3]);
-    const R h = R(itg.h), sqrth = R(itg.sqrth), x0 = R(itg.x), y0 = R(itg.y);
+    const R h = R(itg.h), sqrth = R(itg.sqrth);
+    R x0 = R(itg.x), y0 = R(itg.y);
     const R s0 = R(itg.sub[0]), s1 = R(itg.sub[1]), s2 = R(itg.sub[2]), s3 = R(itg.sub[3]);
     const bool has_sub = (ST != 0) || itg.sub_shape >= 0;
     const bool sub_circle = (ST == 1) || (ST == 0 && itg.sub_shape == 1);
-    // A subdomain strictly inside the rectangular domain is always nearer (in
-    // Dentro's signed distance) than the domain boundary, wherever the path
-    // is, so the domain distance cannot decide an exit and is not evaluated.
-    bool dom_can_win = true;
-    if (has_sub && DomainOf<PROB>::shape == 0) {
-      if (sub_circle)  // (r, cx, cy)
-        dom_can_win = !(s1 - s0 > d0 && s1 + s0 < d2 && s2 - s0 > d1 && s2 + s0 < d3);
-      else             // (x0, y0, x1, y1)
-        dom_can_win = !(s0 > d0 && s1 > d1 && s2 < d2 && s3 < d3);
-    }
-    const R st0 = Problem<PROB>::template state<R>(bvp, x0, y0);  // sigma state at the start point
-    const R sg0 = Problem<PROB>::template sigma_of<R>(st0);
-    // FP64 stepping (kLean): the exit test of Dentro with few FP64
-    // instructions, which bound it (one takes 64 issue slots here).  A path
-    // goes on iff every boundary's signed distance is below the (negative)
-    // threshold, so the distances alone are formed, from centres and half
-    // sides kept here; a circle's test compares squared radii, without the
-    // square root.  Dentro's choice of boundary, projection and normal follow
-    // only when some lane of the warp stops.
-    constexpr bool kLean = std::is_same<R, double>::value && !RobinOf<PROB>::value;
-    R dcx = R(0), dcy = R(0), dhx = R(0), dhy = R(0), scx = R(0), scy = R(0), shx = R(0), shy = R(0);
-    if constexpr (kLean) {
-      if constexpr (DomainOf<PROB>::shape == 0) {
-        dcx = R(0.5) * (d0 + d2); dcy = R(0.5) * (d1 + d3); dhx = d2 - dcx; dhy = d3 - dcy;
-      }
-      if (!sub_circle) {
-        scx = R(0.5) * (s0 + s2); scy = R(0.5) * (s1 + s3); shx = s2 - scx; shy = s3 - scy;
-      }
-    }
+    const bool dom_can_win = domain_can_win<PROB>(has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3);
+    R st0 = Problem<PROB>::template state<R>(bvp, x0, y0);  // sigma state at the start point
+    R sg0 = Problem<PROB>::template sigma_of<R>(st0);
+    constexpr bool kLean = std::is_same<R, double>::value && !RobinOf<PROB>::value;  // FP64 stepping: ExitTest
+    [[maybe_unused]] typename std::conditional<kLean, ExitTest<PROB>, NoExitTest>::type test(dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, 0.0);
     // Reflecting sides (FK_PROBLEM_ROBIN), only where the domain can win
     // Dentro's comparison.
     int rmask = 0;
@@ -675,7 +887,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       rphi = R(bvp.prob[1]);
       rho = R(bvp.prob[2]);
     }
-    const uint32_t item = static_cast<uint32_t>(ch.item);
+    uint32_t item = static_cast<uint32_t>(ch.item);  // the lane's item (one for all lanes unless chunks stream)
     // learned control variate: grad u_hat table of this item's region
     const float2* ctab = nullptr;
     R cx0 = R(0), cy0 = R(0), csx = R(0), csy = R(0);
@@ -727,6 +939,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     if (!WM && lane == 0) base = atomicAdd(&sl.next, 32u);
     unsigned pl = __shfl_sync(kFull, base, 0) + lane;
     bool active = pl < n_ch;
+    unsigned path = p0 + pl;  // (its path number; without streaming it is formed from pl where it is used)
     if (cv_table && active) cv_grad(x, y, cgx, cgy);
     int qn = 0;  // queued exits of this warp (warp-uniform)
 
@@ -737,33 +950,90 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       const int qb = qn - cnt;
       const bool mine = lane < cnt;
       R ex = R(0), ey = R(0), Yv = R(0);
+      [[maybe_unused]] R score = R(0), vr = R(0), bv = R(0), xq = R(0);
+      [[maybe_unused]] unsigned kfq = 0;
+      [[maybe_unused]] bool late = false;
       bool sub_exit = false;
+      [[maybe_unused]] int eit = 0;  // the exit's item
       if (mine) {
         const int e = qb + lane;
         ex = q.x[e]; ey = q.y[e]; Yv = q.Y[e];
         const R Zv = q.Z[e], xv = CV ? q.xi[e] : R(0);
         const unsigned kf = q.kf[e];
-        const bool dw = (kf >> 30) & 1u, cp = (kf >> 31) & 1u;
+        bool dw = (kf >> 30) & 1u;
+        const bool cp = (kf >> 31) & 1u;
+        if constexpr (kLean) {
+          // the boundary and the projection, for 32 stopped paths at once
+          Bnd<R> w;
+          dentro_exit<PROB>(ex, ey, dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, w, dw);
+          ex = w.ex;
+          ey = w.ey;
+        }
         sub_exit = (ST != 0) && !dw;
         const R g = Problem<PROB>::u(bvp, ex, ey);  // g = u for every registered problem
-        const R score = Zv + Yv * g;
-        const R vr = score + xv;
-        acc[0].add(score);
-        acc[1].add(score * score);
-        if constexpr (CV) {
-          acc[2].add(xv + xv * xv);
-          acc[3].add(vr);
-          acc[4].add(vr * vr);
-          acc[5].add(xv * score);
-          acc[6].add(sub_exit ? Zv + xv : vr);
-          acc[7].add(xv * xv);
-        } else {  // xi = 0: the VR sums equal the plain ones
-          acc[6].add(sub_exit ? Zv : score);
+        score = Zv + Yv * g;
+        vr = score + xv;
+        if constexpr (kMix) {
+          xq = xv;
+          kfq = (kf & ~(1u << 30)) | (dw ? 1u << 30 : 0u);
         }
-        n_steps += kf & 0x3fffffffu;
-        n_dom += dw ? 1u : 0u;
-        n_cap += cp ? 1u : 0u;
-        ++n_done;
+        bv = sub_exit ? Zv + xv : vr;
+        bool own = true;
+        if constexpr (kMix) {
+          eit = q.it[e];
+          own = eit == cur;
+          late = !own;
+        }
+        if (__builtin_expect(own, 1)) {
+          acc[0].add(score);
+          acc[1].add(score * score);
+          if constexpr (CV) {
+            acc[2].add(xv + xv * xv);
+            acc[3].add(vr);
+            acc[4].add(vr * vr);
+            acc[5].add(xv * score);
+            acc[7].add(xv * xv);
+          }  // (otherwise xi = 0: the VR sums equal the plain ones)
+          acc[6].add(bv);
+          n_steps += kf & 0x3fffffffu;
+          n_dom += dw ? 1u : 0u;
+          n_cap += cp ? 1u : 0u;
+          ++n_done;
+        }
+      }
+      if constexpr (kMix) {
+        // paths of earlier chunks that outlived them: to their items' sums, one item at a time
+        unsigned lm = __ballot_sync(kFull, late);
+        while (__builtin_expect(lm != 0u, 0)) {
+          const int one = __shfl_sync(kFull, eit, __ffs(lm) - 1);
+          const bool sel = late && eit == one;
+          lm &= ~__ballot_sync(kFull, sel);
+          AccD la[kNumAcc];
+          unsigned long long ls = 0;
+          unsigned ld = 0, lc = 0, ln = 0;
+          if (sel) {
+            la[0].add(score);
+            la[1].add(score * score);
+            if constexpr (CV) {
+              la[2].add(xq + xq * xq);
+              la[3].add(vr);
+              la[4].add(vr * vr);
+              la[5].add(xq * score);
+              la[7].add(xq * xq);
+            }
+            la[6].add(bv);
+            ls = kfq & 0x3fffffffu;
+            ld = (kfq >> 30) & 1u;
+            lc = (kfq >> 31) & 1u;
+            ln = 1;
+          }
+          add_item_sums<CV>(a, one, la, ls, ld, lc, ln, lane);
+        }
+      }
+      // the exits' stencil moments: the item's accumulators
+      SAcc* eacc = sacc;
+      if constexpr (kMix && ST == 2) {
+        if (a.mix && mine) eacc = reinterpret_cast<SAcc*>(a.acc + a.items[eit].acc_off);
       }
       if (ST == 2) {
         if (sub_exit) {
@@ -789,12 +1059,12 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
             const R dx = ex - snx[idx], dy = ey - sny[idx];
             const R arg = e2 * (dx * dx + dy * dy);
             if (!(arg < R(std::is_same<R, float>::value ? kPhiCut32 : kPhiCut))) return false;
-            const R wv = Yv * fexp(-arg);
+            const R wv = Yv * fexp(bvp.tab, -arg);
             if constexpr (WM && std::is_same<R, float>::value) {
               if (wms) atomicAdd(&wacc[L * kk + j], wv);     // the warp's FP32 moments in shared memory
-              else atomicAdd(&sacc[L * kk + j], f32_to_f64(wv));  // the item's FP64 accumulator in global memory
+              else atomicAdd(&eacc[L * kk + j], f32_to_f64(wv));  // the item's FP64 accumulator in global memory
             } else
-              atomicAdd(&sacc[L * kk + j], static_cast<SAcc>(wv));
+              atomicAdd(&eacc[L * kk + j], static_cast<SAcc>(wv));
             return true;
           };
           if (sp.walk == kWalkSpan && jn < kk) {
@@ -821,14 +1091,24 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         unsigned em = __ballot_sync(kFull, sub_exit);
         const int n = sarc.n;
         const double c2 = sarc.c2;
-        while (em) {
-          const int src = __ffs(em) - 1;
-          em &= em - 1;
-          const double tb = __shfl_sync(kFull, th, src);
-          const double Yb = static_cast<double>(__shfl_sync(kFull, Yv, src));
-          for (int i = lane; i < n; i += 32) {
-            const double d = tb - sth[i];
-            atomicAdd(reinterpret_cast<double*>(&sacc[i]), Yb / sqrt(d * d + c2));
+        if constexpr (kMix) {
+          // the exits of one item summed in registers, then added once
+          while (em) {
+            const int one = __shfl_sync(kFull, eit, __ffs(em) - 1);
+            unsigned im = __ballot_sync(kFull, sub_exit && eit == one);
+            em &= ~im;
+            add_arc_moments(a.acc + a.items[one].acc_off, im, th, static_cast<double>(Yv), sth, n, c2, lane);
+          }
+        } else {
+          while (em) {
+            const int src = __ffs(em) - 1;
+            em &= em - 1;
+            const double tb = __shfl_sync(kFull, th, src);
+            const double Yb = static_cast<double>(__shfl_sync(kFull, Yv, src));
+            for (int i = lane; i < n; i += 32) {
+              const double d = tb - sth[i];
+              atomicAdd(reinterpret_cast<double*>(&sacc[i]), Yb / sqrt(d * d + c2));
+            }
           }
         }
       }
@@ -839,13 +1119,73 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     // steps; queued exits are processed 32 at a time and, once the chunk is
     // exhausted for this warp, the remainder.
     for (;;) {
-      const bool any = __any_sync(kFull, active);
-      if (!any && qn == 0) break;
+      // lanes that found the chunk's paths all taken: does the next chunk join?
+      bool join = false;
+      ChunkDev nc = ch;
+      if constexpr (kMix) if (__builtin_expect(!stop && wnext > n_ch, 0)) {
+        nxt = __shfl_sync(kFull, ahead, 0);
+        stop = true;
+        if (nxt < (CLS ? slots[warp].cls_hi : n_chunks)) {
+          nc = a.chunks[nxt];
+          const ItemDev& ni = a.items[nc.item];
+          bool same = ni.h == itg.h && ni.bvp == itg.bvp && ni.stencil == itg.stencil && ni.cv_region == itg.cv_region &&
+                      ni.sub_shape == itg.sub_shape;
+          if (ST == 0 && itg.sub_shape >= 0)
+            for (int i = 0; i < 4; ++i) same = same && ni.sub[i] == itg.sub[i];
+          if (same) {
+            join = true;
+            stop = false;
+          }
+        }
+      }
+      bool any = __any_sync(kFull, active);
+      const bool leave = !any && qn == 0 && !join;
+      if (__builtin_expect(leave || (join && nc.item != cur), 0)) {
+        // ---- the warp leaves the item: its sums into the item's FP64 sums
+        add_item_sums<CV>(a, cur, acc, n_steps, n_dom, n_cap, n_done, lane);
+        if (leave) break;
+#pragma unroll
+        for (int j = 0; j < kNumAcc; ++j) acc[j] = Acc();
+        n_steps = 0;
+        n_dom = n_cap = n_done = 0;
+      }
+      if constexpr (kMix) if (__builtin_expect(join, 0)) {
+        if (nc.item != cur) {
+          const ItemDev& ni = a.items[nc.item];
+          x0 = R(ni.x);
+          y0 = R(ni.y);
+          st0 = Problem<PROB>::template state<R>(bvp, x0, y0);
+          sg0 = Problem<PROB>::template sigma_of<R>(st0);
+          cur = nc.item;
+        }
+        const unsigned taken = n_ch;
+        p0 = nc.p0;
+        n_ch = nc.p1 - nc.p0;
+        wnext -= taken;
+        if (!active) {  // (every idle lane holds a path number from `taken` on)
+          pl -= taken;
+          active = pl < n_ch;
+          path = p0 + pl;
+          item = static_cast<uint32_t>(cur);
+          x = x0; y = y0; Y = R(1); Z = R(0); xi = R(0); k = 0; st = st0; sgc = sg0;
+          if (cv_table && active) cv_grad(x, y, cgx, cgy);
+        }
+        nxt = -1;
+        if (lane == 0) ahead = atomicAdd(CLS ? slots[warp].cls_next : a.queue, 1);
+        any = __any_sync(kFull, active);
+      }
       bool exits = false, dom_wins = true, capped = false;
       R ex = R(0), ey = R(0);
       if (active) {
         // ---- one Euler-Maruyama step (Paso_Absorbente, FeynmanKacSolver.cpp:7-18)
         StepCoef<R> co;
+        R z0, z1;
+        if constexpr (kLean) {
+          // (the normals before the coefficients: independent work in one
+          // branch-free stretch, whose long integer chains overlap)
+          const uint4 rl = philox10_rk(make_uint4(static_cast<uint32_t>(k), kMix ? path : ch.p0 + pl, item, a.stream), a.rkey);
+          box_muller(bvp.tab, rl.x, rl.y, z0, z1);
+        }
         Problem<PROB>::step(bvp, x, y, st, sgc, cv_exact, co);
         if (cv_table) {
           // F = -sigma^T grad u_hat at the step's start point, looked up
@@ -857,10 +1197,10 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         // x and y: every lane computes a block at every step, so the warp
         // stays converged (a block split over two steps put the lanes' step
         // parities, and with them the Philox branch, out of step)
-        const uint4 r = philox10_rk(make_uint4(static_cast<uint32_t>(k), ch.p0 + pl, item, a.stream), a.rkey);
-        const uint32_t wa = r.x, wb = r.y;
-        R z0, z1;
-        box_muller(wa, wb, z0, z1);
+        if constexpr (!kLean) {
+          const uint4 r = philox10_rk(make_uint4(static_cast<uint32_t>(k), kMix ? path : ch.p0 + pl, item, a.stream), a.rkey);
+          box_muller(bvp.tab, r.x, r.y, z0, z1);
+        }
         if constexpr (kLean) {
           // the Euler step with the terms that are zero for the problem left out
           const R sh = co.s * sqrth;
@@ -901,7 +1241,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
               const R dq = q == 0 ? d0 - x : (q == 1 ? d1 - y : (q == 2 ? x - d2 : y - d3));
               if (!(dq > -rho)) continue;
               if (!drawn) {
-                re = philox10_rk(make_uint4(0x80000000u | static_cast<uint32_t>(k), ch.p0 + pl, item, a.stream),
+                re = philox10_rk(make_uint4(0x80000000u | static_cast<uint32_t>(k), kMix ? path : ch.p0 + pl, item, a.stream),
                                  a.rkey);
                 drawn = true;
               }
@@ -959,25 +1299,15 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
             st = Problem<PROB>::template state<R>(bvp, x, y);
             sgc = Problem<PROB>::template sigma_of<R>(st);
           }
-          const R thr = R(kGobet) * (sgc * sqrth);
-          // d < thr < 0 of a rectangle: the larger of two negative offsets, as integers
-          auto rect_in = [&](R cx, R cy, R hx, R hy) {
-            const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
-            // (a negative double grows as its bits fall; a non-negative or NaN offset fails the comparison)
-            return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
-          };
-          auto circle_in = [&](R r0, R cx, R cy) {  // |x - c|, at least 5e-4, below r0 + thr
-            const R nx = x - cx, ny = y - cy, rho = r0 + thr;
-            return rho > R(5e-4) && nx * nx + ny * ny < rho * rho;
-          };
-          bool in = true;
-          if (dom_can_win)
-            in = DomainOf<PROB>::shape == 1 ? circle_in(d0, d1, d2) : rect_in(dcx, dcy, dhx, dhy);
-          if (has_sub) in = in && (sub_circle ? circle_in(s0, s1, s2) : rect_in(scx, scy, shx, shy));
+          test.thr = R(kGobet) * (sgc * sqrth);
+          const bool in = test.inside(x, y);
           capped = k >= a.max_steps;
           exits = !in || capped;
         }
-        if (!kLean || exits) {
+        if constexpr (kLean) {
+          ex = x;  // (Dentro's boundary follows when the queued exits are processed)
+          ey = y;
+        } else {
         Bnd<R> w;
         if (dom_can_win) {
           w = (DomainOf<PROB>::shape == 1) ? circle_dist<R>(x, y, d0, d1, d2) : rect_dist<R>(x, y, d0, d1, d2, d3);
@@ -989,7 +1319,6 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           w = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
           dom_wins = false;
         }
-        if constexpr (!kLean) {
         // sigma at the new point (kept for the next step) or at the
         // projection: one evaluation at the selected point, no divergence
         const bool inside = w.d < R(0);
@@ -1050,7 +1379,6 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
             sgc = Problem<PROB>::template sigma_of<R>(st);
           }
         }
-        }
         ex = w.ex;
         ey = w.ey;
         }
@@ -1072,8 +1400,13 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           const int e = qn + rank;
           q.x[e] = ex; q.y[e] = ey; q.Y[e] = Y; q.Z[e] = Z; if constexpr (CV) q.xi[e] = xi;
           q.kf[e] = static_cast<unsigned>(k) | (dom_wins ? 1u << 30 : 0u) | (capped ? 1u << 31 : 0u);
+          if constexpr (kMix) {
+            q.it[e] = static_cast<int>(item);
+            item = static_cast<uint32_t>(cur);
+          }
           pl = nb + rank;
           active = pl < n_ch;
+          if constexpr (kMix) path = p0 + pl;
           x = x0; y = y0; Y = R(1); Z = R(0); xi = R(0); k = 0; st = st0; sgc = sg0;
         }
         qn += __popc(em);
@@ -1088,32 +1421,6 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       }
     }
 
-    // ---- the warp leaves the chunk: its sums into the item's FP64 sums
-    double* sums = a.stats + static_cast<long long>(ch.item) * kNumStats;
-    const int slot_of[kNumAcc] = {kStatScore, kStatScore2, kStatXiAlias, kStatVR,
-                                  kStatVR2, kStatXiScore, kStatB, kStatXi2};
-#pragma unroll
-    for (int j = 0; j < kNumAcc; ++j) {
-      if (!CV && j != 0 && j != 1 && j != 6) continue;
-      const double t = warp_reduce(acc[j], lane);
-      if (lane == 0 && t != 0.0) {
-        atomicAdd(&sums[slot_of[j]], t);
-        if (!CV && j < 2) atomicAdd(&sums[slot_of[j + 3]], t);  // score -> VR, score^2 -> VR^2
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      n_steps += __shfl_xor_sync(kFull, n_steps, o);
-      n_dom += __shfl_xor_sync(kFull, n_dom, o);
-      n_cap += __shfl_xor_sync(kFull, n_cap, o);
-      n_done += __shfl_xor_sync(kFull, n_done, o);
-    }
-    if (lane == 0) {
-      if (n_steps) atomicAdd(&sums[kStatSteps], static_cast<double>(n_steps));
-      if (n_dom) atomicAdd(&sums[kStatDom], static_cast<double>(n_dom));
-      if (n_cap) atomicAdd(&sums[kStatCap], static_cast<double>(n_cap));
-      if (n_done) atomicAdd(&sums[kStatPaths], static_cast<double>(n_done));
-    }
     __syncwarp();
     if (WM) {
       if constexpr (kWmsCapable) {
@@ -1168,24 +1475,35 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
 }
 
 // The kernel instantiation of a launch: stencil kind st (0 points, 1 arcs,
-// 2 patches), `four` the 4-CTA build of FP32 patch slot mode; CV: the build
-// with the control-variate terms (without them xi = 0 and the VR sums are the
-// plain ones).
+// 2 patches), `alt` the 4-CTA build of FP32 patch slot mode or the build of
+// point solves with several classes of chunks; CV: the build with the
+// control-variate terms (without them xi = 0 and the VR sums are the plain
+// ones).
 template <typename R, int PROB, bool WM, bool CV>
-const void* paths_fn(int st, bool four) {
+const void* paths_fn(int st, bool alt) {
   constexpr int MB = std::is_same<R, double>::value ? 2 : 3;
+  constexpr bool CLS = WM && std::is_same<R, double>::value;  // (stencils that stream: as many classes as stencils)
   switch (st) {
-    case 1: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 1, WM, MB, CV>);
+    case 1: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 1, WM, MB, CV, CLS>);
     case 2:
       if constexpr (std::is_same<R, float>::value && !WM)
-        if (four) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, 4, CV>);
-      return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV>);
-    default: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, WM, MB, CV>);
+        if (alt) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, 4, CV, false>);
+      return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV, CLS>);
+    default:
+      if constexpr (std::is_same<R, double>::value) {
+        // FP64 point solves have no stencil moments to share: always warp mode
+        if constexpr (WM)
+          return alt ? reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, true>)
+                     : reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, false>);
+        return nullptr;
+      } else {
+        return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, WM, MB, CV, false>);
+      }
   }
 }
 template <typename R, bool WM, bool CV>
-const void* paths_fn_r(int problem, int st, bool four) {
-  return with_problem(problem, [&](auto t) { return paths_fn<R, decltype(t)::value, WM, CV>(st, four); });
+const void* paths_fn_r(int problem, int st, bool alt) {
+  return with_problem(problem, [&](auto t) { return paths_fn<R, decltype(t)::value, WM, CV>(st, alt); });
 }
 
 }  // namespace

@@ -7,12 +7,12 @@
 
 namespace fk {
 
-const void* select_paths_plain(int problem, int precision, int st, bool warp_mode, bool four) {
+const void* select_paths_plain(int problem, int precision, int st, bool warp_mode, bool alt) {
   if (precision == 1)
-    return warp_mode ? paths_fn_r<float, true, false>(problem, st, false)
-                     : paths_fn_r<float, false, false>(problem, st, four);
-  return warp_mode ? paths_fn_r<double, true, false>(problem, st, false)
-                   : paths_fn_r<double, false, false>(problem, st, false);
+    return warp_mode ? paths_fn_r<float, true, false>(problem, st, alt)
+                     : paths_fn_r<float, false, false>(problem, st, alt);
+  return warp_mode ? paths_fn_r<double, true, false>(problem, st, alt)
+                   : paths_fn_r<double, false, false>(problem, st, alt);
 }
 
 }  // namespace fk

@@ -20,7 +20,7 @@ int main() {
   ld e = 0;
   auto try_exp = [&](double v) {
     const ld x = expl((ld)v);
-    e = fmaxl(e, fabsl((ld)exp_core(v) - x) / x * 9007199254740992.0L);
+    e = fmaxl(e, fabsl((ld)exp_core(tables(), v) - x) / x * 9007199254740992.0L);
   };
   for (int i = 0; i < 1000000; ++i) try_exp(-100 + 110 * U(rng));
   for (int i = 0; i < 200000; ++i) try_exp((U(rng) - 0.5) * std::ldexp(1.0, -(i % 60)));
@@ -35,7 +35,7 @@ int main() {
   e = 0;
   auto try_log = [&](u32 a) {
     int ex;
-    const u64 l = neg_log(a, ex);
+    const u64 l = neg_log(tables(), a, ex);
     e = fmaxl(e, fabsl(l * ldexpl(1, ex - 1) + logl(((ld)a + 0.5L) * ldexpl(1, -32))));
   };
   for (int i = 0; i < 1000000; ++i) try_log((u32)rng());
@@ -51,7 +51,7 @@ int main() {
   e = 0;
   auto try_sc = [&](u32 b) {
     u64 c, s;
-    sincos_quadrant(b, c, s);
+    sincos_quadrant(tables(), b, c, s);
     const ld t = 2 * pi * ((ld)(b & 0x3fffffffu) + 0.5L) * ldexpl(1, -32);
     e = fmaxl(e, fmaxl(fabsl(c * ldexpl(1, -63) - cosl(t)), fabsl(s * ldexpl(1, -63) - sinl(t))));
   };
@@ -75,23 +75,27 @@ int main() {
   put("sqrt_ulp", e);
   // normal pair: absolute, and the FP64 forms' beside it
   e = 0;
-  ld f = 0, e2 = 0, f2 = 0;
+  ld f = 0, e2 = 0, f2 = 0, efx = 0;
   const int n = 1000000;
   for (int i = 0; i < n; ++i) {
     const u32 a = i < 64 ? (i < 32 ? 1u << i : ~(1u << (i - 32))) : (u32)rng(), b = (u32)rng();
     double z0, z1;
-    normal_pair(a, b, z0, z1);
+    normal_pair(tables(), a, b, z0, z1);
     const ld u1 = ((ld)a + 0.5L) * ldexpl(1, -32), u2 = ((ld)b + 0.5L) * ldexpl(1, -32), r = sqrtl(-2 * logl(u1));
     const ld x0 = r * cosl(2 * pi * u2), x1 = r * sinl(2 * pi * u2);
     const double du1 = (a + 0.5) * 2.3283064365386962890625e-10, du2 = (b + 0.5) * 2.3283064365386962890625e-10;
     const double dr = std::sqrt(-2.0 * std::log(du1));
     const ld d0 = dr * std::cos(6.283185307179586 * du2), d1 = dr * std::sin(6.283185307179586 * du2);
+    i64 k0, k1;
+    normal_pair_fx(tables(), a, b, k0, k1);
+    efx = fmaxl(efx, fmaxl(fabsl(k0 * ldexpl(1, -53) - x0), fabsl(k1 * ldexpl(1, -53) - x1)));
     const ld m = fmaxl(fabsl(z0 - x0), fabsl(z1 - x1)), k = fmaxl(fabsl(d0 - x0), fabsl(d1 - x1));
     e = fmaxl(e, m);
     f = fmaxl(f, k);
     e2 += m * m;
     f2 += k * k;
   }
+  put("normal_fx_abs", efx);
   put("normal_abs", e);
   put("normal_abs_fp64", f);
   put("normal_rms", sqrtl(e2 / n));
@@ -132,14 +136,14 @@ int main() {
     FrankeArgs fa;
     FrankeTerms ft;
     franke_args(X, Y, fa);
-    franke_terms(fa, ft);
+    franke_terms(tables(), fa, ft);
     i64 ux, uy, gx, gy;
     franke_grad(fa, ft, ux, uy);
-    const u64 a62 = aniso_a(X, Y);
+    const u64 a62 = aniso_a(tables(), X, Y);
     AnisoOut o;
-    aniso_step(X, Y, a62, o);
+    aniso_step(tables(), X, Y, a62, o);
     aniso_grad(X, Y, o, gx, gy);
-    const ld v[11] = {to_double(franke_lap(fa), -54), to_double(franke_u(ft), -60), ux * ldexpl(1, -58), uy * ldexpl(1, -58),
+    const ld v[11] = {to_double(franke_lap(tables(), fa), -54), to_double(franke_u(ft), -60), ux * ldexpl(1, -58), uy * ldexpl(1, -58),
                       franke_lap_terms(fa, ft) * ldexpl(1, -54), to_double(a62, 0u, -62), aniso_sigma(a62), to_double(o.f, -51),
                       to_double(o.mc, 0u, -54), gx * ldexpl(1, -54), gy * ldexpl(1, -54)};
     const ld e[11] = {E.lap, E.u, E.ux, E.uy, E.lap, E.a, E.s, E.f, E.mc, E.Ux, E.Uy};

@@ -19,10 +19,11 @@ def errors(tmp_path_factory):
 
 
 @pytest.mark.parametrize("name,bound", [
-    ("exp_ulp", 1.75),            # units of 2^-53: the result's rounding 1, the exponent 2 units of 2^-54 times ln 2
+    ("exp_ulp", 1.3),             # units of 2^-53: the result's rounding 1, the exponent's 2^-55 1/4, products 2^-58
     ("neg_log_abs", 2.0 ** -55),  # 16 units of 2^-59
     ("sincos_abs", 2.0 ** -58),   # theta^5 / 120 at theta = pi / 4096, and products low by 2 units of 2^-63
     ("sqrt_ulp", 2.0 ** -4),      # units of 2^-53: 2^-57
+    ("normal_fx_abs", 2.0 ** -53),  # rounding to 2^-53 units, and the pair's own 2^-54 at |z| up to 6.8
 ])
 def test_bounds(errors, name, bound):
     assert errors[name][0] <= bound

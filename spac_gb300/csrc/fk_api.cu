@@ -647,9 +647,11 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // mode: every warp takes its own chunks and adds the stencil moments to
   // global memory, so an item's slowest path holds up one warp only.  A
   // launch shape set by the caller (fk_set_launch, the autotuner) keeps the
-  // shared chunk slots, but for FP64 point solves, which have no stencil
-  // moments to share and always run in warp mode.
-  bool warp_mode = (kind == 0 && precision == FK_FP64) || (ctx->chunk <= 0 && n_live > 0 && total_paths <= kWarpModeMaxPaths * n_live);
+  // shared chunk slots, but for point solves, which have no stencil moments
+  // to share and always run in warp mode.
+  const bool few = ctx->chunk <= 0 && n_live > 0 && total_paths <= kWarpModeMaxPaths * n_live;
+  bool warp_mode = kind == 0 || few;
+  const bool stream = precision == FK_FP64 || (kind == 0 && !few);  // (of warp mode: warps go from chunk to chunk undrained)
   // Adaptive rounds with items of few paths: warp mode with per-warp FP32
   // moment accumulators in shared memory, so that the kernel forms the G rows
   // (the rounds keep no moments in global memory).  CTAs of 4 warps (2 for
@@ -668,24 +670,26 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     }
   }
   if (round && warp_mode && !wms) warp_mode = false;  // (rounds need rows formed in the kernel)
-  const size_t sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
+  size_t sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
+  if (sacc_bytes > 200 * 1024 && warp_mode && precision == FK_FP64 && lblock > 32) {  // (room for the tables: fewer warps)
+    lblock = std::max(32, lblock / 64 * 32);
+    sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
+  }
   if (sacc_bytes > 200 * 1024) return fail(ctx, FK_ERR_CAPACITY, "stencil accumulators exceed shared memory");
-  int occ = fk::paths_kernel_occupancy(bvp.problem, precision, kind, any_cv ? 1 : 0, lblock, sacc_bytes, warp_mode);
-  // (the 3 CTAs per SM that FP32 slot builds are sized for, also where one needs fewer registers)
-  if (kind == 0 && precision == FK_FP32 && !warp_mode && lblock == 256) occ = std::min(occ, 3);
+  const int occ = fk::paths_kernel_occupancy(bvp.problem, precision, kind, any_cv ? 1 : 0, lblock, sacc_bytes, warp_mode, stream);
   int grid = std::max(1, ctx->num_sms * occ);
   int block_used = lblock;
   size_t smem_used = sacc_bytes;
   int group = 1;  // lanes per path
   if (warp_mode && ctx->chunk <= 0 && bvp.cv != FK_CV_MLP && fk::paths_group_available(bvp.problem, precision, kind))
     group = group_width(ctx, it);
-  const bool mix = warp_mode && group == 1 && precision == FK_FP64;
+  const bool mix = warp_mode && group == 1 && stream;
   if (group > 1) {
     // as many warps per SM as there are paths for, up to 16 (two CTAs)
     const long long want = (total_paths * group + 32LL * ctx->num_sms - 1) / (32LL * ctx->num_sms);
     block_used = static_cast<int>(32 * std::max<long long>(1, std::min<long long>(8, want)));
     grid = ctx->num_sms * (want > 8 ? 2 : 1);
-  } else if (mix && ctx->chunk <= 0 && block == 256) {
+  } else if (mix && ctx->chunk <= 0 && lblock == 256) {
     // Streaming: full occupancy from 4 paths per lane on; with fewer paths
     // fewer warps, whose lanes stay busy longer, but one per scheduler at
     // least (37 anisotropic points x 1,501 paths: 4.0 ms on 4 warps per SM, 4.7
@@ -720,9 +724,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     chunk = std::max<long long>(std::max<long long>(kind == 1 ? 32 : ng, total_paths >> 20), std::min(chunk, 32 * ng));
   } else if (mix && chunk <= 0) {
     // Streaming: 64 to 512 paths, about 32 chunks per warp for point solves
-    // (1,024 points x 10^4 paths: 14.9 ms at 64 paths, 15.0 at 128, 16.7 at
-    // 512; but the host lists every chunk, 8 ms for 88 M paths in pieces of
-    // 128) and 8 with a stencil (8x8 FP64 assembly: 15.6 ms at 512,
+    // (1,024 points x 10^4 paths in FP64: 14.9 ms at 64 paths, 15.0 at 128,
+    // 16.7 at 512; 16 uneven disks in FP32: 46.1 at 128, 48.2 at 512, but the
+    // host lists every chunk, 8 ms for 88 M paths in pieces of 128) and 8 with
+    // a stencil (8x8 FP64 assembly: 15.6 ms at 512,
     // 15.9 at 128); never more than 2^20 chunks.
     chunk = total_paths / ((kind == 0 ? 32LL : 8LL) * grid * (block_used / 32));
     chunk = std::max<long long>(std::max<long long>(64, total_paths >> 20), std::min<long long>(chunk, 512));

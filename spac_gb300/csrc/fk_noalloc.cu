@@ -242,9 +242,8 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return FK_ERR_CUDA;
   const int block = 256;
   const int cvm = (d->cv == FK_CV_EXACT) ? 1 : 0;
-  const bool warp_mode = precision == FK_FP64;  // (as fk_solve_points: FP64 point solves stream in warp mode)
-  const size_t smem = paths_smem_bytes(precision, 0, 0, 0, warp_mode, block);
-  const int grid = sms * paths_kernel_occupancy(d->problem, precision, 0, cvm, block, smem, warp_mode);
+  const size_t smem = paths_smem_bytes(precision, 0, 0, 0, true, block);
+  const int grid = sms * paths_kernel_occupancy(d->problem, precision, 0, cvm, block, smem, true, true);
   // the work counter, the status words and the FP64 sums start at zero on every call
   if (cudaMemsetAsync(d_queue, 0, 4 * sizeof(int), s) != cudaSuccess) return FK_ERR_CUDA;
   if (cudaMemsetAsync(d_stats, 0, sizeof(double) * kNumStats * n, s) != cudaSuccess) return FK_ERR_CUDA;
@@ -269,9 +268,9 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   a.cv = cvm;
   a.any_cv = d->cv != FK_CV_NONE ? 1 : 0;
   a.stencil_kind = 0;
-  a.mix = warp_mode ? 1 : 0;
+  a.mix = 1;
   a.n_cls = 1;
-  if (launch_paths(a, d->problem, precision, grid, block, smem, s, warp_mode) != cudaSuccess) return FK_ERR_CUDA;
+  if (launch_paths(a, d->problem, precision, grid, block, smem, s, true) != cudaSuccess) return FK_ERR_CUDA;
 
   FinalizeArgs f;
   std::memset(&f, 0, sizeof(f));

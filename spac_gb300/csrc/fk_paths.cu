@@ -18,7 +18,7 @@ const void* select_paths_v(int problem, int precision, int st, bool warp_mode, b
 }
 // The variant a launch uses: the 4-CTA build for FP32 patch-stencil slot
 // mode when 4 of its CTAs fit on an SM with this shared memory and block.
-const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv, int n_cls) {
+const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv, bool mode2) {
   if (precision == 1 && st == 2 && !warp_mode && block == 256) {
     const void* f4 = select_paths_v(problem, precision, st, warp_mode, true, cv);
     int n = 0;
@@ -27,7 +27,7 @@ const void* select_paths(int problem, int precision, int st, bool warp_mode, int
       return f4;
     cudaGetLastError();
   }
-  return select_paths_v(problem, precision, st, warp_mode, st == 0 && n_cls > 1, cv);
+  return select_paths_v(problem, precision, st, warp_mode, st == 0 && mode2, cv);
 }
 
 }  // namespace
@@ -43,15 +43,16 @@ size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block, size_t smem,
                          cudaStream_t s, bool warp_mode) {
   if (block < 32 || block > 256 || block % 32 != 0) return cudaErrorInvalidValue;
-  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0, a.n_cls);
+  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0, a.mix && (precision == 1 || a.n_cls > 1));
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<LaunchArgs*>(&a)};
   return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, s);
 }
 
-int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem, bool warp_mode) {
-  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0, 1);
+int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem, bool warp_mode,
+                           bool stream) {
+  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0, stream);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess) return 1;

@@ -113,20 +113,16 @@ struct PatchSh {
   R knn_u0[4];
 };
 
-// Streaming (FP64 warp mode): the warp's class of chunks (its index, end and
-// counter) and the classes it has not been in, kept out of the registers of the
-// step loop.
-template <typename R>
-struct ClassSh {};
-template <>
-struct ClassSh<double> {
+// Streaming: the warp's class of chunks (its index, end and counter) and the
+// classes it has not been in, kept out of the registers of the step loop.
+struct ClassSh {
   int cls, cls_hi, cls_left;
   int* cls_next;
 };
 
 // A chunk slot.  `ready` is written last, after the slot's contents.
 template <typename R>
-struct SlotSh : ClassSh<R> {
+struct SlotSh {
   int ready;        // position in the CTA's chunk sequence that the slot holds
   int chunk;        // chunk index; -1: the chunk queue was exhausted
   int warps_left;   // warps that have not yet left the chunk
@@ -701,20 +697,20 @@ __device__ __forceinline__ void add_arc_moments(double* acc, unsigned im, double
 // admits 4 CTAs: it runs the 8x8 assembly 2.9 % faster, while point solves,
 // warp mode and the larger patches of the 32x32 mesh measured slower at 64
 // registers.
-// CLS: streaming with more than one class of chunks.  Point solves also have a
-// build without: the class bookkeeping, though it runs once per chunk, costs
-// the step loop 12 to 18 % of its latency (one point x 1,000 paths: 0.53
-// against 0.46 ms), and most calls have one class.
-template <typename R, int PROB, int ST, bool WM, int MB, bool CV, bool CLS>
+// MODE (warp mode): 0 the warp drains at the end of every chunk; 1 streaming
+// (below); 2 streaming with several classes of chunks.  FP64 always streams;
+// FP32 only in point solves of many paths per item: its thread sums round to
+// 2^-24 of a path's score at every addition, so another partition of the paths
+// moves a mean of a few hundred by 4e-9, and its stencil launches form their
+// rows per item in the kernel.  Mode 1 is for FP64 point solves of one class:
+// the class bookkeeping, though it runs once per chunk, costs the step loop 12
+// to 18 % of its latency (one point x 1,000 paths: 0.53 against 0.46 ms).
+template <typename R, int PROB, int ST, bool WM, int MB, bool CV, int MODE>
 __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
   using SAcc = typename std::conditional<WM, double, typename SAccType<R, ST>::type>::type;
   using Acc = typename std::conditional<std::is_same<R, double>::value, AccD, AccK>::type;
   constexpr int kPrec = std::is_same<R, double>::value ? 0 : 1;
-  // streaming builds (below): FP64 stepping.  FP32 keeps its chunks apart: its
-  // thread sums round to 2^-24 of a path's score at every addition, so another
-  // partition of the paths moves a mean of a few hundred paths by 4e-9, and its
-  // stencil launches of warp mode form their rows per item in the kernel.
-  constexpr bool kMix = WM && std::is_same<R, double>::value;
+  constexpr bool kMix = MODE > 0, CLS = MODE == 2;
   // FP64 stepping in warp mode: the function tables at the start of the shared memory
   constexpr bool kShTab = WM && kPrec == 0;
   constexpr size_t kTab = kShTab ? sizeof(fx::Tables) : 0;
@@ -722,6 +718,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SlotSh<R> slots[S];
   __shared__ ExitQueue<R, kMix> sq[kMaxBlockWarps];
+  __shared__ ClassSh classes[kMix ? kMaxBlockWarps : 1];
   // warp mode with per-warp FP32 moment accumulators in shared memory (FP32
   // patch stencils): the warp forms its chunk's G row itself when it leaves
   constexpr bool kWmsCapable = WM && ST == 2 && std::is_same<R, float>::value;
@@ -759,7 +756,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
   int ahead = -1, nxt = -1;
   if constexpr (kMix) {
     if (lane == 0) {
-      SlotSh<R>& w = slots[warp];
+      ClassSh& w = classes[warp];
       w.cls = 0;
       w.cls_left = 1;
       w.cls_hi = n_chunks;
@@ -787,7 +784,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       nxt = -1;
       if constexpr (kMix) {
         if (lane == 0) {
-          SlotSh<R>& w = slots[warp];
+          ClassSh& w = classes[warp];
           while (CLS && c >= w.cls_hi && --w.cls_left > 0) {  // the class has run out: the next one's
             w.cls = w.cls + 1 < a.n_cls ? w.cls + 1 : 0;
             w.cls_hi = a.cls_first[w.cls + 1];
@@ -1125,7 +1122,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
       if constexpr (kMix) if (__builtin_expect(!stop && wnext > n_ch, 0)) {
         nxt = __shfl_sync(kFull, ahead, 0);
         stop = true;
-        if (nxt < (CLS ? slots[warp].cls_hi : n_chunks)) {
+        if (nxt < (CLS ? classes[warp].cls_hi : n_chunks)) {
           nc = a.chunks[nxt];
           const ItemDev& ni = a.items[nc.item];
           bool same = ni.h == itg.h && ni.bvp == itg.bvp && ni.stencil == itg.stencil && ni.cv_region == itg.cv_region &&
@@ -1171,7 +1168,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           if (cv_table && active) cv_grad(x, y, cgx, cgy);
         }
         nxt = -1;
-        if (lane == 0) ahead = atomicAdd(CLS ? slots[warp].cls_next : a.queue, 1);
+        if (lane == 0) ahead = atomicAdd(CLS ? classes[warp].cls_next : a.queue, 1);
         any = __any_sync(kFull, active);
       }
       bool exits = false, dom_wins = true, capped = false;
@@ -1475,30 +1472,27 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
 }
 
 // The kernel instantiation of a launch: stencil kind st (0 points, 1 arcs,
-// 2 patches), `alt` the 4-CTA build of FP32 patch slot mode or the build of
-// point solves with several classes of chunks; CV: the build with the
+// 2 patches), `alt` the 4-CTA build of FP32 patch slot mode or the mode 2
+// build of point solves; CV: the build with the
 // control-variate terms (without them xi = 0 and the VR sums are the plain
 // ones).
 template <typename R, int PROB, bool WM, bool CV>
 const void* paths_fn(int st, bool alt) {
-  constexpr int MB = std::is_same<R, double>::value ? 2 : 3;
-  constexpr bool CLS = WM && std::is_same<R, double>::value;  // (stencils that stream: as many classes as stencils)
+  constexpr bool f64 = std::is_same<R, double>::value;
+  constexpr int MB = f64 ? 2 : 3;
+  constexpr int MODE = WM && f64 ? 2 : 0;  // (stencils that stream: as many classes as stencils)
   switch (st) {
-    case 1: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 1, WM, MB, CV, CLS>);
+    case 1: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 1, WM, MB, CV, MODE>);
     case 2:
-      if constexpr (std::is_same<R, float>::value && !WM)
-        if (alt) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, 4, CV, false>);
-      return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV, CLS>);
+      if constexpr (!f64 && !WM)
+        if (alt) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, 4, CV, 0>);
+      return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV, MODE>);
     default:
-      if constexpr (std::is_same<R, double>::value) {
-        // FP64 point solves have no stencil moments to share: always warp mode
-        if constexpr (WM)
-          return alt ? reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, true>)
-                     : reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, false>);
-        return nullptr;
-      } else {
-        return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, WM, MB, CV, false>);
-      }
+      // point solves have no stencil moments to share: always warp mode
+      if constexpr (WM)
+        return alt ? reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, 2>)
+                   : reinterpret_cast<const void*>(&paths_kernel<R, PROB, 0, true, MB, CV, f64 ? 1 : 0>);
+      return nullptr;
   }
 }
 template <typename R, bool WM, bool CV>

@@ -58,6 +58,10 @@ struct DiskDev {
   long long inner_off;  // first interior node of the disk (in the batch)
   long long g_off;      // first G entry (n_inner x n_periph)
   long long periph_off; // first periphery angle
+  // the first disk of the batch with the same radial tables and mode
+  // eigenvalues, and the first with the same grid angles and periphery angles
+  // (this disk's own index if there is none before it)
+  int op_rep, ring_rep;
 };
 
 // Host-side batch: tables shared by disks of equal (radius, N_radio) and N_c.

@@ -117,3 +117,25 @@ def test_patch_stencil_streaming_rows(gpu, fk, precision):
     tol = 1e-11 if precision == "FP64" else 2e-6
     for k in ("val", "B", "item_G", "item_B"):
         assert np.allclose(out[0][k], out[1][k], rtol=tol, atol=tol), k
+
+
+@pytest.mark.parametrize("problem", [0, 2])
+def test_disk_rows_shared_operators(gpu, fk, problem):
+    """A batch whose disks share radii, grids and periphery angles in part gives
+    each disk the rows that it gets alone, bit for bit."""
+    rng = np.random.default_rng(3)
+    disks = []
+    for i in range(12):
+        nc, r, t0 = (16, 20)[i % 3 == 2], (0.1, 0.17)[i % 2], (0.1, 0.3)[i % 4 == 3]
+        c = rng.uniform(0.3, 0.7, 2)
+        th = t0 + 2 * np.pi * np.arange(nc) / nc
+        if i == 7:
+            th = th + 1e-3
+        rr, aa = 0.9 * r * np.sqrt(rng.random(5)), 2 * np.pi * rng.random(5)
+        disks.append(dict(cx=c[0], cy=c[1], radius=r, theta0=t0, n_circle=nc, n_radial=(11, 13)[i % 5 == 4], periph_theta=th,
+                          inner_xy=np.stack([c[0] + rr * np.cos(aa), c[1] + rr * np.sin(aa)], 1)))
+    b = gpu.register_bvp(problem)
+    batch = gpu.solve_disks_ps(b, disks)
+    for d, (G, B) in zip(disks, batch):
+        (g, v), = gpu.solve_disks_ps(b, [d])
+        assert np.array_equal(G, g) and np.array_equal(B, v)

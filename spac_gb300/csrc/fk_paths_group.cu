@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256, 2) paths_group_kernel(const LaunchArgs a)
     const bool dom_can_win = domain_can_win<PROB>(has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3);
     const R sg = Problem<PROB>::template sigma_of<R>(R(0));
     const R sh = sg * sqrth;
-    const ExitTest<PROB> test(dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, R(kGobet) * sh);
+    const ExitTest<R, PROB> test(dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, R(kGobet) * sh);
     // (1 + c h)^gl and (1 + c h)^G
     StepCoef<R> co;
     R pw = R(1), pwG = R(1), pw1 = R(1);

@@ -589,39 +589,51 @@ __device__ __forceinline__ void dentro_exit(R x, R y, bool dom_can_win, bool has
   }
 }
 
-// FP64 stepping: the exit test of Dentro with few FP64 instructions (one
-// takes 64 issue slots here).  A path goes on iff every boundary's signed
-// distance is below the (negative) threshold, so the distances alone are
-// formed, from centres and half sides kept here; a circle's test compares
-// squared radii, without the square root.  Dentro's choice of boundary,
-// projection and normal follow only when some lane of the warp stops.
-template <int PROB>
+// The exit test of Dentro.  A path goes on iff every boundary's signed
+// distance is below the (negative) threshold, so a step forms the distances
+// alone, from centres and half sides kept here; Dentro's choice of boundary,
+// projection and normal follow for 32 stopped paths at once.  FP64 stepping
+// (one FP64 instruction takes 64 issue slots here) orders the offsets as
+// integers and compares a circle's squared radii, without the square root;
+// FP32 stepping decides on the distances Dentro forms, to the last bit.
+template <typename R, int PROB>
 struct ExitTest {
+  static constexpr bool k64 = std::is_same<R, double>::value;
   bool dom, sub, circle;
-  double dcx, dcy, dhx, dhy, scx, scy, shx, shy, thr;
-  __device__ __forceinline__ ExitTest(bool dom_can_win, bool has_sub, bool sub_circle, double d0, double d1, double d2, double d3,
-                                      double s0, double s1, double s2, double s3, double thr_)
-      : dom(dom_can_win), sub(has_sub), circle(sub_circle), dcx(d1), dcy(d2), dhx(d0), dhy(0.0), scx(s1), scy(s2), shx(s0),
-        shy(0.0), thr(thr_) {
+  R dcx, dcy, dhx, dhy, scx, scy, shx, shy, thr;
+  __device__ __forceinline__ ExitTest(bool dom_can_win, bool has_sub, bool sub_circle, R d0, R d1, R d2, R d3, R s0, R s1, R s2,
+                                      R s3, R thr_)
+      : dom(dom_can_win), sub(has_sub), circle(sub_circle), dcx(d1), dcy(d2), dhx(d0), dhy(R(0)), scx(s1), scy(s2), shx(s0),
+        shy(R(0)), thr(thr_) {
     if (DomainOf<PROB>::shape == 0) {
-      dcx = 0.5 * (d0 + d2); dcy = 0.5 * (d1 + d3); dhx = d2 - dcx; dhy = d3 - dcy;
+      dcx = R(0.5) * (d0 + d2); dcy = R(0.5) * (d1 + d3); dhx = d2 - dcx; dhy = d3 - dcy;
     }
     if (!sub_circle) {
-      scx = 0.5 * (s0 + s2); scy = 0.5 * (s1 + s3); shx = s2 - scx; shy = s3 - scy;
+      scx = R(0.5) * (s0 + s2); scy = R(0.5) * (s1 + s3); shx = s2 - scx; shy = s3 - scy;
     }
   }
-  // d < thr < 0 of a rectangle: the larger of two negative offsets, as integers (a
-  // negative double grows as its bits fall; a non-negative or NaN offset fails)
-  __device__ __forceinline__ bool rect_in(double x, double y, double cx, double cy, double hx, double hy) const {
-    const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
-    return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
+  __device__ __forceinline__ bool rect_in(R x, R y, R cx, R cy, R hx, R hy) const {
+    if constexpr (k64) {
+      // d < thr < 0: the larger of two negative offsets, as integers (a negative
+      // double grows as its bits fall; a non-negative or NaN offset fails)
+      const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
+      return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
+    } else {
+      // (the form of the comparisons: rect_dist of a NaN abscissa is the other offset)
+      const R ox = fabs(x - cx) - hx, oy = fabs(y - cy) - hy;
+      return oy < thr && !(ox >= thr);
+    }
   }
-  // |x - c|, at least 5e-4, below r0 + thr
-  __device__ __forceinline__ bool circle_in(double x, double y, double r0, double cx, double cy) const {
-    const double nx = x - cx, ny = y - cy, rho = r0 + thr;
-    return rho > 5e-4 && nx * nx + ny * ny < rho * rho;
+  __device__ __forceinline__ bool circle_in(R x, R y, R r0, R cx, R cy) const {
+    if constexpr (k64) {
+      // |x - c|, at least 5e-4, below r0 + thr
+      const R nx = x - cx, ny = y - cy, rho = r0 + thr;
+      return rho > 5e-4 && nx * nx + ny * ny < rho * rho;
+    } else {
+    return circle_dist<R>(x, y, r0, cx, cy).d < thr;
+    }
   }
-  __device__ __forceinline__ bool inside(double x, double y) const {
+  __device__ __forceinline__ bool inside(R x, R y) const {
     bool in = true;
     if (dom) in = DomainOf<PROB>::shape == 1 ? circle_in(x, y, dhx, dcx, dcy) : rect_in(x, y, dcx, dcy, dhx, dhy);
     if (sub) in = in && (circle ? circle_in(x, y, shx, scx, scy) : rect_in(x, y, scx, scy, shx, shy));
@@ -873,8 +885,16 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
     const bool dom_can_win = domain_can_win<PROB>(has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3);
     R st0 = Problem<PROB>::template state<R>(bvp, x0, y0);  // sigma state at the start point
     R sg0 = Problem<PROB>::template sigma_of<R>(st0);
-    constexpr bool kLean = std::is_same<R, double>::value && !RobinOf<PROB>::value;  // FP64 stepping: ExitTest
-    [[maybe_unused]] typename std::conditional<kLean, ExitTest<PROB>, NoExitTest>::type test(dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, 0.0);
+    // ExitTest in the step, Dentro's projection in process().  FP32 stepping does so
+    // with patch stencils, whose boundaries are rectangles: 11.29 -> 11.02 ms for
+    // the 8 x 8 assembly, 4.71 -> 4.53 ms with a learned variate.  Where a boundary
+    // may be a circle the whole of circle_dist stays in the step: the compiler
+    // contracts its sums by their surroundings, and the projection rounds
+    // differently in process() (8e-9 of a mean over 64 paths).
+    constexpr bool kLean = !RobinOf<PROB>::value && (kPrec == 0 || (DomainOf<PROB>::shape == 0 && ST == 2));
+    constexpr bool kLean64 = kLean && kPrec == 0;
+    [[maybe_unused]] typename std::conditional<kLean, ExitTest<R, PROB>, NoExitTest>::type test(
+        dom_can_win, has_sub, sub_circle, d0, d1, d2, d3, s0, s1, s2, s3, R(0));
     // Reflecting sides (FK_PROBLEM_ROBIN), only where the domain can win
     // Dentro's comparison.
     int rmask = 0;
@@ -1177,7 +1197,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         // ---- one Euler-Maruyama step (Paso_Absorbente, FeynmanKacSolver.cpp:7-18)
         StepCoef<R> co;
         R z0, z1;
-        if constexpr (kLean) {
+        if constexpr (kLean64) {
           // (the normals before the coefficients: independent work in one
           // branch-free stretch, whose long integer chains overlap)
           const uint4 rl = philox10_rk(make_uint4(static_cast<uint32_t>(k), kMix ? path : ch.p0 + pl, item, a.stream), a.rkey);
@@ -1194,11 +1214,11 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
         // x and y: every lane computes a block at every step, so the warp
         // stays converged (a block split over two steps put the lanes' step
         // parities, and with them the Philox branch, out of step)
-        if constexpr (!kLean) {
+        if constexpr (!kLean64) {
           const uint4 r = philox10_rk(make_uint4(static_cast<uint32_t>(k), kMix ? path : ch.p0 + pl, item, a.stream), a.rkey);
           box_muller(bvp.tab, r.x, r.y, z0, z1);
         }
-        if constexpr (kLean) {
+        if constexpr (kLean64) {
           // the Euler step with the terms that are zero for the problem left out
           const R sh = co.s * sqrth;
           Z += TraitsOf<PROB>::no_potential ? co.f * h : (co.f * Y) * h;
@@ -1216,7 +1236,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           y += sh * z1;
         }
         const R dWx = sqrth * z0, dWy = sqrth * z1;
-        if constexpr (kLean) {
+        if constexpr (kLean64) {
         } else if constexpr (RobinOf<PROB>::value) {
           // ---- Paso_Reflejante (FeynmanKacSolver.cpp:19-67) on reflecting sides
           R xn = x + (co.bx * h + co.s * dWx), yn = y + (co.by * h + co.s * dWy);
@@ -1296,7 +1316,7 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
             st = Problem<PROB>::template state<R>(bvp, x, y);
             sgc = Problem<PROB>::template sigma_of<R>(st);
           }
-          test.thr = R(kGobet) * (sgc * sqrth);
+          test.thr = kLean64 ? R(kGobet) * (sgc * sqrth) : R(kGobet) * sgc * sqrth;
           const bool in = test.inside(x, y);
           capped = k >= a.max_steps;
           exits = !in || capped;

@@ -624,8 +624,8 @@ struct RobinOf<4> {
 // problem's constant c (paths_group_kernel forms a path's steps in parallel).
 template <int PROB>
 struct TraitsOf {
-  static constexpr bool const_sigma = PROB != 2 && PROB != 4;
-  static constexpr bool no_drift = PROB != 2 && PROB != 4;
+  static constexpr bool const_sigma = PROB == 0 || PROB == 1 || PROB == 3 || PROB == 5;
+  static constexpr bool no_drift = const_sigma;
   static constexpr bool no_potential = PROB == 0 || PROB == 3 || PROB == 5;
 };
 
@@ -634,8 +634,9 @@ struct TraitsOf {
 // (include/spac_fk.h).  To add one: write its Problem<N> (state, sigma_of,
 // step and u as above, all for both stepping types; psi and a RobinOf<N>
 // specialisation if it has reflecting sides; a DomainOf<N> specialisation if
-// its domain is a circle; a TraitsOf<N> specialisation if sigma, drift or
-// potential are not as the default says), give it FK_PROBLEM_ value N = kNumProblems and
+// its domain is a circle; a TraitsOf<N> specialisation if its FP64 stepping is
+// to gain from a constant sigma or potential or from no drift: the default
+// claims none of them), give it FK_PROBLEM_ value N = kNumProblems and
 // raise kNumProblems.  with_problem then instantiates and dispatches every
 // kernel (paths, finalize, disk rows) for it; the registry accepts it and
 // checks its domain shape.

@@ -11,11 +11,13 @@
 // CTA-wide barrier between chunks, so the tail of one chunk overlaps the
 // next.  The last warp to leave a chunk flushes the chunk's stencil moments
 // into the item's FP64 accumulators and refills the slot from the global
-// chunk queue.  Items of few paths run in warp mode instead: each warp takes
-// its own chunks and adds the moments to global memory (see paths_kernel).
+// chunk queue.  Items of few paths, all FP64 point solves and FP32 point
+// solves of many paths run in warp mode instead: each warp takes its own
+// chunks and adds the moments to global memory; FP64 stepping and the FP32
+// point solves of many paths stream from chunk to chunk (see paths_kernel).
 //
-// An exiting lane only pushes its exit (X_tau, Y, Z, xi, steps, flags) onto
-// its warp's shared-memory queue and starts the next path; once 32 exits are
+// An exiting lane only pushes its exit (X_tau, or the point it stopped at
+// where the projection follows later, Y, Z, xi, steps, flags) onto its warp's shared-memory queue and starts the next path; once 32 exits are
 // queued the whole warp processes them, one exit per lane, so the exit work
 // runs at full SIMD width:
 //  - exit value u(X_tau), B and the statistics into per-thread registers
@@ -694,8 +696,10 @@ __device__ __forceinline__ void add_arc_moments(double* acc, unsigned im, double
   if (lane + 32 < n) atomicAdd(&acc[lane + 32], m1);
 }
 
-// FP64 stepping is bound by the FP64 pipe, not by latency: it trades
-// occupancy for registers (2 CTAs of 256 per SM instead of 3).
+// FP64 stepping is bound by instruction issue and the latency of its 64-bit
+// integer chains (fk_fixed.cuh; 14 FP64 instructions of a step's 225 are
+// left): it holds whole normals and exponentials in registers and runs 2 CTAs
+// of 256 per SM instead of 3.
 //
 // WM (warp mode, for items of few paths): every warp claims its own chunk
 // from the queue, stages the item's stencil in its own shared-memory

@@ -1,8 +1,7 @@
 // Path-kernel builds without the control-variate terms (xi = 0), for launches
 // whose items all use FK_CV_NONE: five of the eight per-thread compensated
 // sums and the xi state drop out of the step loop.  In FP32 this frees the
-// registers the 4-CTA build otherwise spills; in FP64 it halves the spills of
-// the 2-CTA build (about 3 % of an FP64 assembly).
+// registers the 4-CTA build otherwise spills.
 #include "fk_paths_kernel.cuh"
 
 namespace fk {

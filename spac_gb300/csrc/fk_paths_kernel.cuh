@@ -697,7 +697,7 @@ __device__ __forceinline__ void add_arc_moments(double* acc, unsigned im, double
 }
 
 // FP64 stepping is bound by instruction issue and the latency of its 64-bit
-// integer chains (fk_fixed.cuh; 14 FP64 instructions of a step's 225 are
+// integer chains (fk_fixed.cuh; 10 FP64 instructions of a step's 225 are
 // left): it holds whole normals and exponentials in registers and runs 2 CTAs
 // of 256 per SM instead of 3.
 //

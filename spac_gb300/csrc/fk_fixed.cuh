@@ -66,19 +66,24 @@ FX_FN u64 sqrhi(u64 a) {
   const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a);
   return static_cast<u64>(ah) * ah + ((static_cast<u64>(ah) * al) >> 31);
 }
+// Sums that may wrap (arguments outside a function's range, whose results are not
+// used, and partial sums whose total is in range).
+FX_FN i64 addw(i64 a, i64 b) { return static_cast<i64>(static_cast<u64>(a) + static_cast<u64>(b)); }
+FX_FN i64 subw(i64 a, i64 b) { return static_cast<i64>(static_cast<u64>(a) - static_cast<u64>(b)); }
+FX_FN i64 shlw(i64 a, int k) { return static_cast<i64>(static_cast<u64>(a) << k); }
 // Signed: (a b) >> 64 and (a b) >> S (32 < S < 64) for |a|, |b| < 2^62, low by less than 2 units.
 FX_FN i64 smulhi(i64 a, i64 b) {
   const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
   const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
-  const i64 t = ah * bl + al * bh;
+  const i64 t = addw(ah * bl, al * bh);
   return static_cast<i64>(ah) * bh + (t >> 32);
 }
 template <int S>
 FX_FN i64 smulshr(i64 a, i64 b) {
   const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
   const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
-  const i64 t = ah * bl + al * bh + static_cast<i64>(mulhi32(static_cast<u32>(a), static_cast<u32>(b)));
-  return static_cast<i64>(static_cast<u64>(static_cast<i64>(ah) * bh) << (64 - S)) + (t >> (S - 32));
+  const i64 t = addw(addw(ah * bl, al * bh), static_cast<i64>(mulhi32(static_cast<u32>(a), static_cast<u32>(b))));
+  return addw(shlw(static_cast<i64>(ah) * bh, 64 - S), t >> (S - 32));
 }
 FX_FN int clz64(u64 v) {
 #ifdef __CUDA_ARCH__
@@ -229,7 +234,7 @@ FX_FN double to_double(u64 mag, u32 sign, int e2) {
 }
 FX_FN double to_double(i64 v, int e2) {
   const i64 s = v >> 63;
-  return to_double(static_cast<u64>((v ^ s) - s), static_cast<u32>(s) & 1u, e2);
+  return to_double(static_cast<u64>(subw(v ^ s, s)), static_cast<u32>(s) & 1u, e2);
 }
 
 // -------------------------------------------------------------- exp --------
@@ -421,7 +426,7 @@ FX_FN bool to_pos(double v, i64& p) {
   const bool small = s >= 3;  // |v| < 2
   s = small ? (s < 63 ? s : 63) : 3;
   const i64 sg = static_cast<i64>(b) >> 63;
-  p = (static_cast<i64>(m >> s) ^ sg) - sg;
+  p = subw(static_cast<i64>(m >> s) ^ sg, sg);
   // -3/8 <= p 2^-59 < 11/8
   return small && static_cast<u32>(p >> 32) + 0x03000000u < 0x0E000000u;
 }
@@ -437,19 +442,23 @@ struct FrankeArgs {
 };
 FX_FN u64 abs64(i64 v) {
   const i64 s = v >> 63;
-  return static_cast<u64>((v ^ s) - s);
+  return static_cast<u64>(subw(v ^ s, s));
 }
+// (Unsigned sums: Gx + Gy passes 2^63 near the range's upper corner, and 9x does
+// for the positions outside it, whose results are overwritten.)
 FX_FN void franke_args(i64 X, i64 Y, FrankeArgs& f) {
-  f.X9 = 9 * X;
-  f.Y9 = 9 * Y;
+  f.X9 = static_cast<i64>(9 * static_cast<u64>(X));
+  f.Y9 = static_cast<i64>(9 * static_cast<u64>(Y));
   f.Gx = sqr63(abs64(f.X9)) + 1;
   f.Gy = sqr63(abs64(f.Y9)) + 1;
-  const i64 S = static_cast<i64>(f.Gx + f.Gy + 2);  // (the 2: no sum below falls under zero by rounding)
-  const i64 xq = f.X9 >> 2, xe = f.X9 >> 3, yq = f.Y9 >> 2, ye = f.Y9 >> 3;
-  f.s1 = static_cast<u64>(S - xq - yq) + 8 * kOne55;
-  f.s3 = static_cast<u64>(S - (f.X9 - xe) - (yq + ye)) + 58 * kOne55;
-  f.s4 = static_cast<u64>(S - (f.X9 >> 1) - (f.Y9 - ye)) + 65 * kOne55;
-  f.c2 = f.Gx + 2 + static_cast<u64>(xe) + kOne55;
+  const u64 S = f.Gx + f.Gy + 2;  // (the 2: no sum below falls under zero by rounding)
+  const u64 x9 = static_cast<u64>(f.X9), y9 = static_cast<u64>(f.Y9);
+  const u64 xq = static_cast<u64>(f.X9 >> 2), xe = static_cast<u64>(f.X9 >> 3);
+  const u64 yq = static_cast<u64>(f.Y9 >> 2), ye = static_cast<u64>(f.Y9 >> 3);
+  f.s1 = S - xq - yq + 8 * kOne55;
+  f.s3 = S - (x9 - xe) - (yq + ye) + 58 * kOne55;
+  f.s4 = S - static_cast<u64>(f.X9 >> 1) - (y9 - ye) + 65 * kOne55;
+  f.c2 = f.Gx + 2 + xe + kOne55;
   f.v2 = static_cast<i64>(mulhi(f.c2, 0x14E5E0A72F053978ull) + mulhi(static_cast<u64>(f.Y9 >> 1) + (5ull << 58), 0x0CCCCCCCCCCCCCCDull));
 }
 // Laplacian of the Franke function, 2^-54 units; each coefficient c is folded
@@ -459,11 +468,11 @@ FX_FN i64 franke_lap(const Tables* tb, const FrankeArgs& f) {
   const u64 E1 = exp_neg_fx<57, 59 + 4>(tb, f.s1 + 0x001AAEF2D0FB10FCull), E3 = exp_neg_fx<57, 59 + 4>(tb, f.s3 + 0x00EA481236F7D35Cull);
   const u64 E4 = exp_neg_fx<55, 56 + 7>(tb, f.s4 + 0x005721FC55588EF9ull);
   const u64 E2 = exp_neg_fx<57, 62 - 2>(tb, static_cast<u64>(f.v2) + 0x0102319DC0F73A58ull);
-  i64 l = static_cast<i64>(mulshr<60>(f.s1, E1)) - static_cast<i64>(E1 >> 3);
-  l += static_cast<i64>(mulshr<60>(f.s3, E3)) - static_cast<i64>(E3 >> 3);
-  l -= static_cast<i64>(mulshr<57>(f.s4, E4)) - static_cast<i64>(E4 >> 2);
-  l += static_cast<i64>(mulshr<63>(f.c2, E2)) - static_cast<i64>(mulhi(E2, 0x127F5C28F5C28F5Cull));
-  return l;
+  u64 l = mulshr<60>(f.s1, E1) - (E1 >> 3);
+  l += mulshr<60>(f.s3, E3) - (E3 >> 3);
+  l -= mulshr<57>(f.s4, E4) - (E4 >> 2);
+  l += mulshr<63>(f.c2, E2) - mulhi(E2, 0x127F5C28F5C28F5Cull);
+  return static_cast<i64>(l);
 }
 // b1 = 3/4 e1, b2 = 3/4 e2, b3 = e3 / 2, b4 = e4 / 5, 2^-60 units: u = b1 + b2 + b3 - b4
 struct FrankeTerms {
@@ -481,8 +490,8 @@ FX_FN i64 franke_u(const FrankeTerms& b) { return static_cast<i64>(b.b1 + b.b2 +
 // u_y = 9y (-9/2 (b1 + b3) + 18 b4) + 9 b1 - 9/10 b2 + 27/2 b3 - 126 b4
 FX_FN void franke_grad(const FrankeArgs& f, const FrankeTerms& b, i64& ux, i64& uy) {
   const u64 gb = mulhi(b.b2, 0x2F05397829CBC14Full);  // g b2, 2^-59
-  const i64 wy = static_cast<i64>(9 * b.b4) - static_cast<i64>((9 * ((b.b1 + b.b3) >> 1)) >> 1);  // 2^-59
-  const i64 wx = wy - static_cast<i64>(gb);
+  const i64 wy = static_cast<i64>(9 * b.b4 - ((9 * ((b.b1 + b.b3) >> 1)) >> 1));  // 2^-59
+  const i64 wx = subw(wy, static_cast<i64>(gb));
   const u64 v = 2 * b.b1 + (b.b1 >> 2);
   const u64 vx = v - (gb >> 1) + 8 * b.b3 - (b.b3 >> 3) - 18 * b.b4;
   const u64 vy = v - mulhi(b.b2, 0x399999999999999Aull) + 3 * b.b3 + ((3 * b.b3) >> 3) - 32 * b.b4 + (b.b4 >> 1);
@@ -492,11 +501,11 @@ FX_FN void franke_grad(const FrankeArgs& f, const FrankeTerms& b, i64& ux, i64& 
 // Laplacian from the same terms, 2^-54 units:
 // 81/4 ((s1 - 4) b1 + (s3 - 4) b3) - 324 (s4 - 1) b4 + (g^2 c2 - 9 g + 81/100) b2
 FX_FN i64 franke_lap_terms(const FrankeArgs& f, const FrankeTerms& b) {
-  const i64 p = static_cast<i64>(mulshr<57>(f.s1, b.b1) - b.b1) + static_cast<i64>(mulshr<57>(f.s3, b.b3) - b.b3);  // 2^-58
+  const i64 p = static_cast<i64>(mulshr<57>(f.s1, b.b1) - b.b1 + mulshr<57>(f.s3, b.b3) - b.b3);  // 2^-58
   const i64 p4 = static_cast<i64>(mulshr<55>(f.s4, b.b4) - b.b4);                                                  // 2^-60
-  const i64 p2 = static_cast<i64>(mulshr<60>(mulhi(f.c2, 0x228BACD5ABC4B7D1ull), b.b2)) -
-                 static_cast<i64>(mulhi(b.b2, 0x13F80F0BE96E21DBull));                                             // 2^-55
-  return (2 * p + (p >> 1) + (p >> 5) - ((20 * p4 + (p4 >> 2)) >> 1) + p2) >> 1;
+  const i64 p2 = static_cast<i64>(mulshr<60>(mulhi(f.c2, 0x228BACD5ABC4B7D1ull), b.b2) - mulhi(b.b2, 0x13F80F0BE96E21DBull));  // 2^-55
+  return addw(addw(addw(shlw(p, 1), (p >> 1) + (p >> 5)), p2),
+              -(addw(static_cast<i64>(20 * static_cast<u64>(p4)), p4 >> 2) >> 1)) >> 1;
 }
 
 // -------------------------------------- the anisotropic problem's factors ----
@@ -552,22 +561,23 @@ FX_FN void aniso_step(const Tables* tb, i64 X, i64 Y, u64 a62, AnisoOut& o) {
   o.F = franke_u(b);
   franke_grad(f, b, o.Fx, o.Fy);
   const i64 lap = franke_lap_terms(f, b);
-  const i64 X61 = X << 2, Y61 = Y << 2, a61 = static_cast<i64>(a62 >> 1);
-  o.q = (1ll << 60) + (smulhi(X61, Y61) << 2);
+  const i64 X61 = shlw(X, 2), Y61 = shlw(Y, 2), a61 = static_cast<i64>(a62 >> 1);
+  o.q = addw(1ll << 60, shlw(smulhi(X61, Y61), 2));
   o.mc = (kOne55 + mulhi(f.Gx + f.Gy, 0x0329161F9ADD3C0Dull)) >> 1;
-  const i64 adv = smulhi(Y61 - (1ll << 60), o.Fx) + smulhi((1ll << 60) - X61, o.Fy) - smulhi(static_cast<i64>(o.mc << 5), o.F);  // 2^-55
-  const i64 inner = (smulhi(lap, a61) << 2) + (adv >> 2);                  // 2^-53
+  const i64 adv = subw(addw(smulhi(subw(Y61, 1ll << 60), o.Fx), smulhi(subw(1ll << 60, X61), o.Fy)),
+                       smulhi(static_cast<i64>(o.mc << 5), o.F));         // 2^-55
+  const i64 inner = addw(shlw(smulhi(lap, a61), 2), adv >> 2);             // 2^-53
   const i64 t1 = smulshr<62>(inner, o.q);                                  // 2^-51
-  const i64 g = smulhi(o.Fx, Y61) + smulhi(o.Fy, X61);                     // 2^-55
-  const i64 t2 = smulhi(g << 1, a61) >> 1;                                 // 2 a g, 2^-51
-  const i64 h = smulhi(static_cast<i64>(f.Gy - f.Gx) >> 1, 0x0329161F9ADD3C0Dll) + ((X - Y) >> 6);  // 2^-54
-  const i64 t3 = smulhi(o.F, h << 6) >> 5;                                 // 2^-51
-  o.f = -(t1 + t2 + t3);
+  const i64 g = addw(smulhi(o.Fx, Y61), smulhi(o.Fy, X61));                // 2^-55
+  const i64 t2 = smulhi(shlw(g, 1), a61) >> 1;                             // 2 a g, 2^-51
+  const i64 h = addw(smulhi(static_cast<i64>(f.Gy - f.Gx) >> 1, 0x0329161F9ADD3C0Dll), subw(X, Y) >> 6);  // 2^-54
+  const i64 t3 = smulhi(o.F, shlw(h, 6)) >> 5;                             // 2^-51
+  o.f = subw(0, addw(addw(t1, t2), t3));
 }
 // grad u = grad F q + F (y, x), 2^-54 units
 FX_FN void aniso_grad(i64 X, i64 Y, const AnisoOut& o, i64& ux, i64& uy) {
-  ux = smulhi(o.Fx, o.q) + (smulhi(o.F, Y << 2) >> 3);
-  uy = smulhi(o.Fy, o.q) + (smulhi(o.F, X << 2) >> 3);
+  ux = addw(smulhi(o.Fx, o.q), smulhi(o.F, shlw(Y, 2)) >> 3);
+  uy = addw(smulhi(o.Fy, o.q), smulhi(o.F, shlw(X, 2)) >> 3);
 }
 
 }  // namespace fx

@@ -98,7 +98,7 @@ constexpr u64 kLn2_64 = 0xB17217F7D1CF79ACull;  // ln 2 * 2^64
 constexpr u64 kLn2_59 = 0x058B90BFBE8E7BCDull;  // ln 2 * 2^59
 
 struct alignas(16) LogEntry {
-  u64 ln;   // -ln(c / 2^16) * 2^59
+  u64 ln;   // ln(c / 2^15) * 2^64: 0 in the last interval, next to u = 1
   u64 c;    // reciprocal of the interval's middle, 16 bits
 };
 struct alignas(16) SinCosEntry {
@@ -165,10 +165,10 @@ constexpr Tables make_tables() {
     const u64 d = 1025 + 2 * static_cast<u64>(j);  // middle of the interval: d / 1024
     u64 c = ((1ull << 27) / d + 1) >> 1;           // 2^16 / (d / 1024), rounded
     if (j == 511) c = 1ull << 15;                  // exactly 1/2: -ln u is exact near u = 1
-    // -ln(c / 2^16) = 2 atanh((2^16 - c) / (2^16 + c)), series in 2^64
-    const u64 num = 65536 - c, den = 65536 + c;
+    // ln(c / 2^15) = 2 atanh((c - 2^15) / (c + 2^15)), the series in 2^-65: at most 1/3, and few terms where it is small
+    const u64 num = c - 32768, den = c + 32768;
     u64 x = 0, r = num;
-    for (int b = 0; b < 64; ++b) {
+    for (int b = 0; b < 65; ++b) {
       r <<= 1;
       x <<= 1;
       if (r >= den) {
@@ -176,13 +176,13 @@ constexpr Tables make_tables() {
         x |= 1;
       }
     }
-    const u64 x2 = cmulhi(x, x);
+    const u64 x2 = cmulhi(x, x) >> 2;
     u64 p = x, sum = 0;
     for (int k = 1; k < 60 && p; k += 2) {
       sum += p / k;
       p = cmulhi(p, x2);
     }
-    t.log[j].ln = j == 511 ? kLn2_59 : (sum >> 4) + ((sum >> 3) & 1);  // 2 sum 2^-64 in 2^-59
+    t.log[j].ln = sum;  // 2 sum 2^-65
     t.log[j].c = c;
   }
   return t;
@@ -331,8 +331,11 @@ FX_FN u64 sqrt_norm(u64 L, int e, int& e_out) {
 }
 
 // -------------------------------------------------- normal pair -------------
-// l = -ln((a + 1/2) 2^-32) as l 2^59 (e = -58) or, in the last table cell
-// before u = 1, l 2^69 (e = -68); absolute error below 2^-55, there 2^-66.
+// l = -ln((a + 1/2) 2^-32) as l 2^59 (e = -58), for u >= 1/2 as l 2^64 (e = -63), in the
+// last table cell before u = 1 as l 2^72 (e = -71) and for l < 2^-17 as l 2^80 (e = -79):
+// the error of a radius sqrt(2 l) is that of l over it, and with one unit for
+// all l a radius of 2^-5 has two, one of 2^-11 nine times the error that an FP64
+// logarithm leaves it.
 // Exact argument reduction: u = y 2^(30-n), y c - 1 an integer multiple of 2^-48.
 FX_FN u64 neg_log(const Tables* tb, u32 a, int& e) {
   const u64 m = (static_cast<u64>(a) << 1) | 1u;
@@ -344,16 +347,19 @@ FX_FN u64 neg_log(const Tables* tb, u32 a, int& e) {
   const i64 r = static_cast<i64>((Y >> 31) * c - (1ull << 48));  // (y c - 1) 2^48, |r| < 2^38.1
   const i64 sg = r >> 63;
   const u64 A = static_cast<u64>((r ^ sg) - sg) << 24;  // |r| 2^72
-  const u64 r2 = sqrhi(A);                              // r^2 2^80
+  const u64 r2 = sqrhi(A);                              // r^2 2^80 (exact in the last cell)
   const u32 rh = static_cast<u32>(A >> 32), q = static_cast<u32>(r2 >> 29);  // |r| 2^40, r^2 2^51
   const u32 r4 = mulhi32(q, q);                                              // r^4 2^70
-  const u64 odd = (A >> 3) + ((static_cast<u64>(mulhi32(q, 0x55555555u)) * rh) >> 22) +
-                  (mulhi32(mulhi32(r4, rh), 0x33333334u) >> 9);  // |r| + |r|^3/3 + |r|^5/5
-  const u64 even = (r2 >> 12) + (r4 >> 3);                       // r^2/2 + r^4/4
-  const i64 l1p = ((static_cast<i64>(odd) ^ sg) - sg) - static_cast<i64>(even);  // log1p(r) 2^69
-  const u64 base = static_cast<u64>(n - 30) * kLn2_59 - ln;
-  e = base ? -58 : -68;
-  return base ? base - static_cast<u64>(l1p >> 10) : static_cast<u64>(-l1p);
+  const u64 odd = ((static_cast<u64>(mulhi32(q, 0x55555555u)) * rh) >> 11) +
+                  (static_cast<u64>(mulhi32(mulhi32(r4, rh), 0x33333334u)) << 2);    // |r|^3/3 + |r|^5/5, 2^-80
+  const u64 even = (r2 >> 1) + (static_cast<u64>(r4) << 8);                          // r^2/2 + r^4/4
+  const i64 h = ((static_cast<i64>(odd) ^ sg) - sg) - static_cast<i64>(even);        // log1p(r) - r, 2^-80
+  const i64 l1p = ((static_cast<i64>(A) ^ sg) - sg) + (h >> 8);                      // log1p(r), 2^-72
+  const bool half = n == 31, last = half && ln == 0, tiny = last && A < (1ull << 55);  // (there r < 0)
+  e = tiny ? -79 : (last ? -71 : (half ? -63 : -58));
+  const u64 base = half ? ln : static_cast<u64>(n - 31) * kLn2_59 + (ln >> 5);
+  const u64 l = base - static_cast<u64>(l1p >> (last ? 0 : (half ? 8 : 13)));
+  return tiny ? (A << 8) - static_cast<u64>(h) : l;
 }
 
 // cos and sin of the angle b + 1/2 (of 2^32) within its quadrant, times 2^63;

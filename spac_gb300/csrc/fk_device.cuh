@@ -313,12 +313,12 @@ __device__ __forceinline__ void franke_lap_grad(const fx::Tables* tb, double x, 
     fx::FrankeTerms b;
     fx::i64 gx, gy;
     fx::franke_terms(tb, f, b);
-    fx::franke_grad(f, b, gx, gy);
-    ux = fx::to_double(gx, -58);
-    uy = fx::to_double(gy, -58);
-    lap = fx::to_double(fx::franke_lap_terms(f, b), -54);
+    fx::franke_grad<61>(f, b, gx, gy);
+    ux = fx::to_double(gx, -61);
+    uy = fx::to_double(gy, -61);
+    lap = fx::to_double(fx::franke_lap_terms<56>(f, b), -56);
   } else {
-    lap = fx::to_double(fx::franke_lap(tb, f), -54);
+    lap = fx::to_double(fx::franke_lap<56>(tb, f), -56);
   }
   if (__builtin_expect(!ok, 0)) {
     const FrankeFar F = franke_far(x, y);
@@ -334,7 +334,7 @@ __device__ __forceinline__ double franke_value(const fx::Tables* tb, double x, d
   fx::FrankeTerms b;
   fx::franke_args(X, Y, f);
   fx::franke_terms(tb, f, b);
-  double u = fx::to_double(fx::franke_u(b), -60);
+  double u = fx::to_double(fx::franke_u<62>(b), -62);
   if (__builtin_expect(!ok, 0)) u = franke_far(x, y).u;
   return u;
 }
@@ -494,18 +494,18 @@ struct Problem<2> {
     if constexpr (std::is_same<R, double>::value) {
       fx::i64 X, Y;
       const bool ok = fx::to_pos(x, X) & fx::to_pos(y, Y);
-      fx::AnisoOut p;
+      fx::AnisoParts<55, 59> p;
       fx::aniso_step(b.tab, X, Y, fx::a_bits(a), p);
       o.s = s;
-      o.c = -fx::to_double(p.mc, 0u, -54);
+      o.c = -fx::to_double(p.mc, 0u, -59);
       o.bx = y - 0.5;
       o.by = 0.5 - x;
-      o.f = fx::to_double(p.f, -51);
+      o.f = fx::to_double(p.f, -55);
       if (cv) {
         fx::i64 ux, uy;
-        fx::aniso_grad(X, Y, p, ux, uy);
-        o.Fx = -s * fx::to_double(ux, -54);
-        o.Fy = -s * fx::to_double(uy, -54);
+        fx::aniso_grad<60>(X, Y, p, ux, uy);
+        o.Fx = -s * fx::to_double(ux, -60);
+        o.Fy = -s * fx::to_double(uy, -60);
       }
       if (__builtin_expect(!ok, 0)) o = step_far(x, y, a, s);
     } else {

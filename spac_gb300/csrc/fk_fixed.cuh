@@ -5,10 +5,13 @@
 // written in FP64 is bound by that pipe alone: about 225 such instructions
 // per step for the Franke problem, 3,600 cycles, while the other pipes idle.
 // The functions here compute the step's transcendental and polynomial parts
-// on the integer pipes in 64-bit fixed point, at 52 to 60 fractional bits:
-// no operand, intermediate or result carries less precision than the FP64
-// forms they replace (errors are below, measured against 80-bit arithmetic
-// in tests/cpp/fixed_math_main.cpp).  A 64 x 64 product's upper half is three
+// on the integer pipes in 64-bit fixed point.  Fixed point has absolute units,
+// so a single small operand may hold fewer digits than a double would; units
+// (2^-55 to 2^-80) and the order of products and cuts are chosen so that no
+// result is further off than the FP64 form's, wherever in the range: normals
+// for every size of the radius, source terms in every 1/8 x 1/8 cell of the
+// positions (against long double, tests/cpp/fixed_normals_main.cpp and
+// fixed_cells_main.cpp).  A 64 x 64 product's upper half is three
 // 32 x 32 -> 64 multiply-adds, about 8 of the 64 issue slots that one FP64
 // instruction takes.
 //
@@ -48,18 +51,19 @@ FX_FN u64 mulhi(u64 a, u64 b) {
   t += static_cast<u64>(al) * bh;
   return static_cast<u64>(ah) * bh + (t >> 32);
 }
-// (a b) >> S, 32 < S < 64, for a, b < 2^63 and a result below 2^64, low by less than 2 units.
-template <int S>
+// (a b) >> S, 32 < S < 64, for a < 2^63, b < 2^63 (1 + 2^-19) and a result below 2^64:
+// low by less than 2 units, or (R = 1) rounded to nearest.
+template <int S, int R = 0>
 FX_FN u64 mulshr(u64 a, u64 b) {
   const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a), bh = static_cast<u32>(b >> 32), bl = static_cast<u32>(b);
-  u64 t = static_cast<u64>(ah) * bl + mulhi32(al, bl);
+  u64 t = static_cast<u64>(ah) * bl + (static_cast<u64>(mulhi32(al, bl)) + (static_cast<u64>(R) << (S - 33)));
   t += static_cast<u64>(al) * bh;
   return ((static_cast<u64>(ah) * bh) << (64 - S)) + (t >> (S - 32));
 }
-// a^2 >> 63 for a < 2^63.5, low by less than 2 units.
+// a^2 >> 63 for a < 2^63.5, rounded to nearest.
 FX_FN u64 sqr63(u64 a) {
   const u32 ah = static_cast<u32>(a >> 32), al = static_cast<u32>(a);
-  return ((static_cast<u64>(ah) * ah) << 1) + ((static_cast<u64>(ah) * al + (mulhi32(al, al) >> 1)) >> 30);
+  return ((static_cast<u64>(ah) * ah) << 1) + ((static_cast<u64>(ah) * al + ((mulhi32(al, al) >> 1) + (1u << 29))) >> 30);
 }
 // a^2 >> 64 for a < 2^63, low by less than 2 units.
 FX_FN u64 sqrhi(u64 a) {
@@ -70,19 +74,24 @@ FX_FN u64 sqrhi(u64 a) {
 // used, and partial sums whose total is in range).
 FX_FN i64 addw(i64 a, i64 b) { return static_cast<i64>(static_cast<u64>(a) + static_cast<u64>(b)); }
 FX_FN i64 subw(i64 a, i64 b) { return static_cast<i64>(static_cast<u64>(a) - static_cast<u64>(b)); }
+// v >> K, rounded to nearest
+template <int K>
+FX_FN i64 rshr(i64 v) { return K == 0 ? v : addw(v, (1ll << K) >> 1) >> K; }
 FX_FN i64 shlw(i64 a, int k) { return static_cast<i64>(static_cast<u64>(a) << k); }
-// Signed: (a b) >> 64 and (a b) >> S (32 < S < 64) for |a|, |b| < 2^62, low by less than 2 units.
+// Signed: (a b) >> 64 and (a b) >> S (32 < S < 64) for |a|, |b| < 2^62, low by less than 2 units
+// or (R = 1) rounded to nearest.
 FX_FN i64 smulhi(i64 a, i64 b) {
   const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
   const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
   const i64 t = addw(ah * bl, al * bh);
   return static_cast<i64>(ah) * bh + (t >> 32);
 }
-template <int S>
+template <int S, int R = 0>
 FX_FN i64 smulshr(i64 a, i64 b) {
   const int ah = static_cast<int>(a >> 32), bh = static_cast<int>(b >> 32);
   const i64 al = static_cast<i64>(static_cast<u32>(a)), bl = static_cast<i64>(static_cast<u32>(b));
-  const i64 t = addw(addw(ah * bl, al * bh), static_cast<i64>(mulhi32(static_cast<u32>(a), static_cast<u32>(b))));
+  const i64 t = addw(addw(ah * bl, al * bh), static_cast<i64>(static_cast<u64>(mulhi32(static_cast<u32>(a), static_cast<u32>(b))) +
+                                                                     (static_cast<u64>(R) << (S - 33))));
   return addw(shlw(static_cast<i64>(ah) * bh, 64 - S), t >> (S - 32));
 }
 FX_FN int clz64(u64 v) {
@@ -90,6 +99,26 @@ FX_FN int clz64(u64 v) {
   return __clzll(static_cast<long long>(v));
 #else
   return v ? __builtin_clzll(v) : 64;
+#endif
+}
+
+// v >> k and v << k, 0 for k > 63 and for negative k (the PTX shifts clamp, C++ ones do not)
+FX_FN u64 shr64(u64 v, int k) {
+#ifdef __CUDA_ARCH__
+  u64 r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(k));
+  return r;
+#else
+  return static_cast<u32>(k) > 63u ? 0 : v >> k;
+#endif
+}
+FX_FN u64 shl64(u64 v, int k) {
+#ifdef __CUDA_ARCH__
+  u64 r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(k));
+  return r;
+#else
+  return static_cast<u32>(k) > 63u ? 0 : v << k;
 #endif
 }
 
@@ -258,15 +287,8 @@ FX_FN u64 exp_neg(const Tables* tb, u64 V, int& q) {
   q = static_cast<int>((n + 0xfffffu) >> 20);
   return exp_frac(tb, 0u - n, z);
 }
-// e^-v 2^F, truncated (a result below 2^63).
-template <int U, int F>
-FX_FN u64 exp_neg_fx(const Tables* tb, u64 V) {
-  int q;
-  const u64 M = exp_neg<U>(tb, V, q);
-  const int sh = 62 - F + q;
-  return M >> (sh < 63 ? sh : 63);
-}
-// e^v for |v| < 256, relative error below 1.1 2^-53 (the result's rounding).
+// e^v for |v| < 256, relative error below 1.3 2^-53: the result's rounding, and
+// the exponent's 2^-55.
 FX_FN double exp_core(const Tables* tb, double v) {
   const u64 b = bits_of(v);
   const int e = static_cast<int>(b >> 52) & 0x7ff;
@@ -420,10 +442,18 @@ FX_FN void normal_pair_fx(const Tables* tb, u32 a, u32 b, i64& z0, i64& z1) {
 }
 
 // ------------------------------------------------------ Franke function ----
-// Positions are 2^-59 units.  In [-3/8, 11/8)^2, which holds the unit square
-// and the serial driver's domain, the sums of squares stay below 256 and the
-// slowest exponential above 6e-3, so absolute errors of 2^-50 are relative
-// ones of the same order; elsewhere the FP64 forms run.
+// Positions are 2^-59 units, in [-3/8, 11/8)^2, which holds the unit square and
+// the serial driver's domain: there the sums of squares stay below 256.
+// Elsewhere the FP64 forms run.
+// A sum in fixed point has one absolute error, so it is as exact as the FP64
+// form only if its unit lies below what the smallest sum of the range leaves
+// there, and the factors of an exponential's polynomial (up to 256 of a square,
+// 324 of the Laplacian's e4) must not meet an exponential that was cut to a
+// unit before.  So the products are formed with the exponential's 62 digits,
+// and cut after; results are 2^-56 (Laplacian), 2^-60 (gradient), 2^-62 (value)
+// and 2^-55 units (source of the anisotropic problem).  Worst error of any 1/8
+// x 1/8 cell of the range, in parts of the FP64 form's there (rms): value 0.56,
+// gradient 0.55, Laplacian 0.59, source 0.57 (fixed_cells_main.cpp).
 FX_FN bool to_pos(double v, i64& p) {
   const u64 b = bits_of(v);
   const int e = static_cast<int>(b >> 52) & 0x7ff;
@@ -438,13 +468,13 @@ FX_FN bool to_pos(double v, i64& p) {
 }
 constexpr u64 kOne55 = 1ull << 55;
 // Squares of the four exponents, 2^-55 units.  One square per coordinate:
-// (9x - k)^2 = (9x)^2 - 2k (9x) + k^2, exact sums.
+// (9x - k)^2 = (9x)^2 - 2k (9x) + k^2.
 struct FrankeArgs {
   i64 X9, Y9;       // 9x, 9y (2^-59)
   u64 Gx, Gy;       // (9x)^2, (9y)^2
-  u64 s1, s3, s4;   // a^2 + b^2, p^2 + q^2, r^2 + t^2
+  u64 s1, s3, s4;   // a^2 + b^2, p^2 + q^2, r^2 + t^2 (one unit below zero at the least)
   u64 c2;           // (9x + 1)^2
-  i64 v2;           // (9x + 1)^2 / 49 + (9y + 5) / 10 (2^-57): e2 = e^(4/10 - v2)
+  u64 v2;           // (9x + 1)^2 / 49 + (9y + 5) / 10 (2^-57): e2 = e^(4/10 - v2)
 };
 FX_FN u64 abs64(i64 v) {
   const i64 s = v >> 63;
@@ -455,63 +485,92 @@ FX_FN u64 abs64(i64 v) {
 FX_FN void franke_args(i64 X, i64 Y, FrankeArgs& f) {
   f.X9 = static_cast<i64>(9 * static_cast<u64>(X));
   f.Y9 = static_cast<i64>(9 * static_cast<u64>(Y));
-  f.Gx = sqr63(abs64(f.X9)) + 1;
-  f.Gy = sqr63(abs64(f.Y9)) + 1;
-  const u64 S = f.Gx + f.Gy + 2;  // (the 2: no sum below falls under zero by rounding)
+  f.Gx = sqr63(abs64(f.X9));
+  f.Gy = sqr63(abs64(f.Y9));
+  const u64 S = f.Gx + f.Gy;
   const u64 x9 = static_cast<u64>(f.X9), y9 = static_cast<u64>(f.Y9);
   const u64 xq = static_cast<u64>(f.X9 >> 2), xe = static_cast<u64>(f.X9 >> 3);
   const u64 yq = static_cast<u64>(f.Y9 >> 2), ye = static_cast<u64>(f.Y9 >> 3);
   f.s1 = S - xq - yq + 8 * kOne55;
   f.s3 = S - (x9 - xe) - (yq + ye) + 58 * kOne55;
   f.s4 = S - static_cast<u64>(f.X9 >> 1) - (y9 - ye) + 65 * kOne55;
-  f.c2 = f.Gx + 2 + xe + kOne55;
-  f.v2 = static_cast<i64>(mulhi(f.c2, 0x14E5E0A72F053978ull) + mulhi(static_cast<u64>(f.Y9 >> 1) + (5ull << 58), 0x0CCCCCCCCCCCCCCDull));
+  f.c2 = f.Gx + xe + kOne55;
+  f.v2 = mulhi(f.c2, 0x14E5E0A72F053978ull) + mulhi(static_cast<u64>(f.Y9 >> 1) + (5ull << 58), 0x0CCCCCCCCCCCCCCDull) + 1;
 }
-// Laplacian of the Franke function, 2^-54 units; each coefficient c is folded
+// d M 2^-(S + k): an exponential's polynomial d times the exponential M 2^-k, with
+// the digits of M.  (Large d come with large k: where the product for S = 60 wraps,
+// at d of 64, k is past 63.)
+template <int S>
+FX_FN i64 times_exp(i64 d, u64 M, int k) {
+  const i64 sg = d >> 63;
+  const u64 t = S == 64 ? mulhi(abs64(d), M) : mulshr<S < 64 ? S : 63>(abs64(d), M);
+  const u64 r = shl64(shr64(t, k > 0 ? k : 0), k < 0 ? -k : 0);
+  return subw(static_cast<i64>(r) ^ sg, sg);
+}
+// Laplacian of the Franke function, 2^-U units; each coefficient c is folded
 // into its exponential's exponent as m ln 2 - ln c >= 0, the power of two into its scale:
 // lap = 243/16 (s1 - 4) e1 + 81/8 (s3 - 4) e3 - 324/5 (s4 - 1) e4 + 486/4802 (c2 - 18.4975) e2
+template <int U = 54>
 FX_FN i64 franke_lap(const Tables* tb, const FrankeArgs& f) {
-  const u64 E1 = exp_neg_fx<57, 59 + 4>(tb, f.s1 + 0x001AAEF2D0FB10FCull), E3 = exp_neg_fx<57, 59 + 4>(tb, f.s3 + 0x00EA481236F7D35Cull);
-  const u64 E4 = exp_neg_fx<55, 56 + 7>(tb, f.s4 + 0x005721FC55588EF9ull);
-  const u64 E2 = exp_neg_fx<57, 62 - 2>(tb, static_cast<u64>(f.v2) + 0x0102319DC0F73A58ull);
-  u64 l = mulshr<60>(f.s1, E1) - (E1 >> 3);
-  l += mulshr<60>(f.s3, E3) - (E3 >> 3);
-  l -= mulshr<57>(f.s4, E4) - (E4 >> 2);
-  l += mulshr<63>(f.c2, E2) - mulhi(E2, 0x127F5C28F5C28F5Cull);
-  return static_cast<i64>(l);
+  int q1, q2, q3, q4;
+  const u64 M1 = exp_neg<57>(tb, f.s1 + 0x001AAEF2D0FB10FCull, q1), M3 = exp_neg<57>(tb, f.s3 + 0x00EA481236F7D35Cull, q3);
+  const u64 M4 = exp_neg<55>(tb, f.s4 + 0x005721FC55588EF9ull, q4), M2 = exp_neg<57>(tb, f.v2 + 0x0102319DC0F73A58ull, q2);
+  i64 l = addw(times_exp<64>(static_cast<i64>(f.s1 - 4 * kOne55), M1, q1 - 7),
+               times_exp<64>(static_cast<i64>(f.s3 - 4 * kOne55), M3, q3 - 7));
+  l = subw(l, times_exp<60>(static_cast<i64>(f.s4 - kOne55), M4, q4 - 6));
+  const i64 d2 = static_cast<i64>(f.c2 - 0x093FAE147AE147AEull), sg = d2 >> 63;
+  const i64 t2 = static_cast<i64>(mulshr<63, 1>(abs64(d2), shr64(M2, q2)));
+  return rshr<56 - U>(addw(l, subw(t2 ^ sg, sg)));
 }
-// b1 = 3/4 e1, b2 = 3/4 e2, b3 = e3 / 2, b4 = e4 / 5, 2^-60 units: u = b1 + b2 + b3 - b4
+// b1 = 3/4 e1, b2 = 3/4 e2, b3 = e3 / 2, b4 = e4 / 5 in 2^-63, 2^-62, 2^-64 and 2^-65 units
+// (u = b1 + b2 + b3 - b4), and the Laplacian's parts
+// p = (s1 - 4) b1 + (s3 - 4) b3 (2^-61), p4 = (s4 - 1) b4 (2^-64).
 struct FrankeTerms {
   u64 b1, b2, b3, b4;
+  i64 p, p4;
 };
 FX_FN void franke_terms(const Tables* tb, const FrankeArgs& f, FrankeTerms& b) {
-  b.b1 = exp_neg_fx<57, 60>(tb, f.s1 + 0x00934B1089A6DC94ull);
-  b.b2 = exp_neg_fx<57, 60 + 1>(tb, static_cast<u64>(f.v2) + 0x01296273AC7DAEBAull);
-  b.b3 = exp_neg_fx<57, 59>(tb, f.s3);
-  b.b4 = exp_neg_fx<55, 60 - 2>(tb, f.s4 + 0x001C8FF7C79A9A22ull);
+  int q1, q2, q3, q4;
+  const u64 M1 = exp_neg<57>(tb, f.s1 + 0x00934B1089A6DC94ull, q1), M3 = exp_neg<57>(tb, f.s3 + 0x0162E42FEFA39EF3ull, q3);
+  const u64 M4 = exp_neg<55>(tb, f.s4 + 0x00CE020FBF6C699Bull, q4), M2 = exp_neg<57>(tb, f.v2 + 0x01296273AC7DAEBAull, q2);
+  b.b1 = shr64(M1, q1 - 1) + (shr64(M1, q1 - 2) & 1u);  // (rounded: its last digit counts 54 times in a gradient)
+  b.b2 = shr64(M2, q2 - 1);
+  b.b3 = shr64(M3, q3 - 2);
+  b.b4 = shr64(M4, q4 - 3);
+  b.p = addw(times_exp<64>(static_cast<i64>(f.s1 - 4 * kOne55), M1, q1 - 8),
+             times_exp<64>(static_cast<i64>(f.s3 - 4 * kOne55), M3, q3 - 8));
+  b.p4 = times_exp<60>(static_cast<i64>(f.s4 - kOne55), M4, q4 - 7);
 }
-FX_FN i64 franke_u(const FrankeTerms& b) { return static_cast<i64>(b.b1 + b.b2 + b.b3 - b.b4); }
-// u_x and u_y, 2^-58 units (g = 18/49):
-// u_x = 9x (-9/2 (b1 + b3) - g b2 + 18 b4) + 9 b1 - g b2 + 63/2 b3 - 72 b4
-// u_y = 9y (-9/2 (b1 + b3) + 18 b4) + 9 b1 - 9/10 b2 + 27/2 b3 - 126 b4
+// u, 2^-U units
+template <int U = 60>
+FX_FN i64 franke_u(const FrankeTerms& b) {
+  return rshr<62 - U>(static_cast<i64>((b.b1 >> 1) + b.b2 + (b.b3 >> 2) - (b.b4 >> 3)));
+}
+// u_x and u_y, 2^-U units (g = 18/49):
+// u_x = 9x (18 b4 - 9/2 (b1 + b3) - g b2) + 9 b1 - g b2 + 63/2 b3 - 72 b4
+// u_y = 9y (18 b4 - 9/2 (b1 + b3)) + 9 b1 - 9/10 b2 + 27/2 b3 - 126 b4
+// (sums in 2^-61, whose parts may wrap; below 4 in the end, 3.3 at the most)
+template <int U = 58>
 FX_FN void franke_grad(const FrankeArgs& f, const FrankeTerms& b, i64& ux, i64& uy) {
-  const u64 gb = mulhi(b.b2, 0x2F05397829CBC14Full);  // g b2, 2^-59
-  const i64 wy = static_cast<i64>(9 * b.b4 - ((9 * ((b.b1 + b.b3) >> 1)) >> 1));  // 2^-59
-  const i64 wx = subw(wy, static_cast<i64>(gb));
+  const u64 gb = mulhi(b.b2, 0x5E0A72F05397829Dull);             // g b2, 2^-62
+  const u64 nb = mulhi(b.b2, 0x7333333333333333ull) + 1;         // 9/10 b2, 2^-61
+  // the brackets over 9/2, 2^-63, and 81/2 x, 81/2 y, 2^-55
+  const i64 dy = static_cast<i64>(b.b4 - (b.b1 + ((b.b3 + 1) >> 1)));
+  const i64 dx = subw(dy, static_cast<i64>(mulshr<63, 1>(b.b2, 0x14E5E0A72F053978ull)));
+  const i64 ax = static_cast<i64>(9 * static_cast<u64>(f.X9 >> 3)) >> 2, ay = static_cast<i64>(9 * static_cast<u64>(f.Y9 >> 3)) >> 2;
   const u64 v = 2 * b.b1 + (b.b1 >> 2);
-  const u64 vx = v - (gb >> 1) + 8 * b.b3 - (b.b3 >> 3) - 18 * b.b4;
-  const u64 vy = v - mulhi(b.b2, 0x399999999999999Aull) + 3 * b.b3 + ((3 * b.b3) >> 3) - 32 * b.b4 + (b.b4 >> 1);
-  ux = static_cast<i64>((static_cast<u64>(smulhi(f.X9 >> 1, wx)) << 5) + vx);
-  uy = static_cast<i64>((static_cast<u64>(smulhi(f.Y9 >> 1, wy)) << 5) + vy);
+  const u64 vx = v - (gb >> 1) + 4 * b.b3 - (b.b3 >> 4) - 4 * b.b4 - (b.b4 >> 1);
+  const u64 vy = v - nb + 2 * b.b3 - (b.b3 >> 2) - (b.b3 >> 4) - 8 * b.b4 + (b.b4 >> 3);
+  ux = rshr<61 - U>(addw(smulshr<57, 1>(ax, dx), static_cast<i64>(vx)));
+  uy = rshr<61 - U>(addw(smulshr<57, 1>(ay, dy), static_cast<i64>(vy)));
 }
-// Laplacian from the same terms, 2^-54 units:
-// 81/4 ((s1 - 4) b1 + (s3 - 4) b3) - 324 (s4 - 1) b4 + (g^2 c2 - 9 g + 81/100) b2
+// Laplacian from the same terms, 2^-U units:
+// 81/4 p - 324 p4 + (g^2 c2 - 9 g + 81/100) b2, 81/128 and 81/64 as sums of three halvings
+template <int U = 54>
 FX_FN i64 franke_lap_terms(const FrankeArgs& f, const FrankeTerms& b) {
-  const i64 p = static_cast<i64>(mulshr<57>(f.s1, b.b1) - b.b1 + mulshr<57>(f.s3, b.b3) - b.b3);  // 2^-58
-  const i64 p4 = static_cast<i64>(mulshr<55>(f.s4, b.b4) - b.b4);                                                  // 2^-60
-  const i64 p2 = static_cast<i64>(mulshr<60>(mulhi(f.c2, 0x228BACD5ABC4B7D1ull), b.b2) - mulhi(b.b2, 0x13F80F0BE96E21DBull));  // 2^-55
-  return addw(addw(addw(shlw(p, 1), (p >> 1) + (p >> 5)), p2),
-              -(addw(static_cast<i64>(20 * static_cast<u64>(p4)), p4 >> 2) >> 1)) >> 1;
+  const i64 l = rshr<1>(addw(b.p, addw(b.p >> 2, b.p >> 6))), l4 = addw(b.p4, addw(b.p4 >> 2, b.p4 >> 6));  // 2^-56
+  const i64 k = static_cast<i64>(mulshr<63>(f.c2, 0x451759AB57896FA2ull) - 0x04FE03C2FA5B8877ull);      // 2^-57
+  return rshr<56 - U>(addw(subw(l, l4), smulshr<63, 1>(k, static_cast<i64>(b.b2))));
 }
 
 // -------------------------------------- the anisotropic problem's factors ----
@@ -550,40 +609,45 @@ FX_FN double aniso_sigma(u64 a62) {  // sqrt(2 a)
   const u64 r = sqrt_norm(a62, -61, e);
   return to_double(r, 0u, e);
 }
-// The anisotropic problem at a point: source f (2^-51 units) of
+// The anisotropic problem at a point: source f (2^-UF units) of
 // u = F q, q = 1 + xy, F the Franke function:
 //   f = -(q (a lap F + b . grad F + c F) + 2 a (F_x y + F_y x) + F (y^2 - x^2 + (x - y) / 2)),
-// b = (y - 1/2, 1/2 - x), c = -(1 + x^2 + y^2); and -c (2^-54 units).
-struct AnisoOut {
+// b = (y - 1/2, 1/2 - x), c = -(1 + x^2 + y^2); and -c (2^-UM units).
+template <int UF, int UM>
+struct AnisoParts {
   i64 f;
   u64 mc;
-  i64 F, Fx, Fy, q;  // 2^-60, 2^-58, 2^-58, 2^-60 units
+  i64 F, Fx, Fy, q;  // 2^-61, 2^-60, 2^-60, 2^-60 units
 };
-FX_FN void aniso_step(const Tables* tb, i64 X, i64 Y, u64 a62, AnisoOut& o) {
+typedef AnisoParts<51, 54> AnisoOut;
+template <int UF, int UM>
+FX_FN void aniso_step(const Tables* tb, i64 X, i64 Y, u64 a62, AnisoParts<UF, UM>& o) {
   FrankeArgs f;
   FrankeTerms b;
   franke_args(X, Y, f);
   franke_terms(tb, f, b);
-  o.F = franke_u(b);
-  franke_grad(f, b, o.Fx, o.Fy);
-  const i64 lap = franke_lap_terms(f, b);
+  o.F = franke_u<61>(b);
+  franke_grad<60>(f, b, o.Fx, o.Fy);
+  const i64 lap = franke_lap_terms<55>(f, b);
   const i64 X61 = shlw(X, 2), Y61 = shlw(Y, 2), a61 = static_cast<i64>(a62 >> 1);
-  o.q = addw(1ll << 60, shlw(smulhi(X61, Y61), 2));
-  o.mc = (kOne55 + mulhi(f.Gx + f.Gy, 0x0329161F9ADD3C0Dull)) >> 1;
-  const i64 adv = subw(addw(smulhi(subw(Y61, 1ll << 60), o.Fx), smulhi(subw(1ll << 60, X61), o.Fy)),
-                       smulhi(static_cast<i64>(o.mc << 5), o.F));         // 2^-55
-  const i64 inner = addw(shlw(smulhi(lap, a61), 2), adv >> 2);             // 2^-53
-  const i64 t1 = smulshr<62>(inner, o.q);                                  // 2^-51
-  const i64 g = addw(smulhi(o.Fx, Y61), smulhi(o.Fy, X61));                // 2^-55
-  const i64 t2 = smulhi(shlw(g, 1), a61) >> 1;                             // 2 a g, 2^-51
-  const i64 h = addw(smulhi(static_cast<i64>(f.Gy - f.Gx) >> 1, 0x0329161F9ADD3C0Dll), subw(X, Y) >> 6);  // 2^-54
-  const i64 t3 = smulhi(o.F, shlw(h, 6)) >> 5;                             // 2^-51
-  o.f = subw(0, addw(addw(t1, t2), t3));
+  o.q = addw(1ll << 60, smulshr<62>(X61, Y61));
+  const u64 mc = (1ull << 59) + mulhi((f.Gx + f.Gy) >> 1, 0x6522C3F35BA78195ull);  // 2^-59
+  o.mc = mc >> (59 - UM);
+  const i64 adv = subw(addw(smulshr<63>(subw(Y61, 1ll << 60), o.Fx), smulshr<63>(subw(1ll << 60, X61), o.Fy)),
+                       smulshr<62>(static_cast<i64>(mc), o.F));                // 2^-58
+  const i64 inner = addw(smulshr<61, 1>(lap, a61), rshr<3>(adv));              // 2^-55
+  const i64 t1 = smulshr<60, 1>(inner, o.q);                                   // 2^-55
+  const i64 g = addw(smulshr<63>(o.Fx, Y61), smulshr<63>(o.Fy, X61));          // 2^-58
+  const i64 t2 = smulshr<63, 1>(g, a61);                                       // 2 a g, 2^-55
+  const i64 h = addw(smulshr<61>(static_cast<i64>(f.Gy - f.Gx) >> 1, 0x1948B0FCD6E9E065ll), subw(X, Y));  // 2^-60
+  const i64 t3 = rshr<3>(smulshr<63>(o.F, h));                                 // 2^-55
+  o.f = rshr<55 - UF>(subw(0, addw(addw(t1, t2), t3)));
 }
-// grad u = grad F q + F (y, x), 2^-54 units
-FX_FN void aniso_grad(i64 X, i64 Y, const AnisoOut& o, i64& ux, i64& uy) {
-  ux = addw(smulhi(o.Fx, o.q), smulhi(o.F, shlw(Y, 2)) >> 3);
-  uy = addw(smulhi(o.Fy, o.q), smulhi(o.F, shlw(X, 2)) >> 3);
+// grad u = grad F q + F (y, x), 2^-U units
+template <int U = 54, int UF, int UM>
+FX_FN void aniso_grad(i64 X, i64 Y, const AnisoParts<UF, UM>& o, i64& ux, i64& uy) {
+  ux = rshr<60 - U>(addw(smulshr<60, 1>(o.Fx, o.q), smulshr<62, 1>(o.F, shlw(Y, 2))));
+  uy = rshr<60 - U>(addw(smulshr<60, 1>(o.Fy, o.q), smulshr<62, 1>(o.F, shlw(X, 2))));
 }
 
 }  // namespace fx

@@ -46,14 +46,14 @@ static void fixed(double x, double y, ld (&o)[kFuns]) {
   FrankeTerms ft;
   franke_args(X, Y, fa);
   franke_terms(tables(), fa, ft);
-  GRAD(fa, ft, ux, uy);
+  franke_grad<61>(fa, ft, ux, uy);
   const u64 a62 = aniso_a(tables(), X, Y);
-  ANISO_OUT s;
+  AnisoParts<55, 59> s;
   aniso_step(tables(), X, Y, a62, s);
-  AGRAD(X, Y, s, gx, gy);
-  const ld v[kFuns] = {to_double(FU(ft), -EU), to_double(ux, -EG), to_double(uy, -EG), to_double(FLAP(tables(), fa), -EL),
-                       to_double(FLT(fa, ft), -EL), to_double(a62, 0u, -62), aniso_sigma(a62), to_double(s.f, -EF),
-                       to_double(s.mc, 0u, -EM), to_double(gx, -EA), to_double(gy, -EA)};
+  aniso_grad<60>(X, Y, s, gx, gy);
+  const ld v[kFuns] = {to_double(franke_u<62>(ft), -62), to_double(ux, -61), to_double(uy, -61), to_double(franke_lap<56>(tables(), fa), -56),
+                       to_double(franke_lap_terms<56>(fa, ft), -56), to_double(a62, 0u, -62), aniso_sigma(a62), to_double(s.f, -55),
+                       to_double(s.mc, 0u, -59), to_double(gx, -60), to_double(gy, -60)};
   for (int j = 0; j < kFuns; ++j) o[j] = v[j];
 }
 

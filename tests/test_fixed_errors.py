@@ -23,3 +23,17 @@ def test_normal_pair_by_radius(tmp_path_factory):
     for w in lines:
         rms, top, rms64, top64 = map(float, w[1:])
         assert rms <= rms64 and top <= top64, w
+
+
+def test_problem_functions_by_cell(tmp_path_factory):
+    """Every function in every cell of the range.  Where the last rounding to a
+    double is all of the error on both sides (a, sigma and -c, of order 1), the
+    two rms agree to the noise of 1,500 samples: 1 / sqrt(2 n) = 2 % each."""
+    lines = _lines(tmp_path_factory, "fixed_cells")
+    assert len(lines) == 14 * 14 * 11
+    for w in lines:
+        rms, mean, top, rms64, _, top64 = map(float, w[3:])
+        slack = 1.02 if w[0] in ("a", "sigma", "mc") else 1.0
+        assert rms <= slack * rms64 and top <= slack * top64, w
+        # what does not average out over a path's steps
+        assert abs(mean) <= 0.5 * rms64, w

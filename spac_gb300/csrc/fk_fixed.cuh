@@ -428,17 +428,21 @@ FX_FN void normal_pair(const Tables* tb, u32 a, u32 b, double& z0, double& z1) {
   z0 = to_double(m0, n0, e);
   z1 = to_double(m1, n1, e);
 }
-// The pair in 2^-53 units, rounded to nearest (|z| < 6.8, so e <= -57).
+// One of the pair's parts in 2^-U units, rounded to nearest (|z| < 6.8, so e <= -57; U <= 55).
+template <int U>
+FX_FN i64 normal_fx(u64 m, u32 n, int e) {
+  const int s = -U - e < 63 ? -U - e : 63;
+  const i64 k = -static_cast<i64>(n);
+  return (static_cast<i64>((m + (1ull << (s - 1))) >> s) ^ k) - k;
+}
+template <int U = 53>
 FX_FN void normal_pair_fx(const Tables* tb, u32 a, u32 b, i64& z0, i64& z1) {
   u64 m0, m1;
   u32 n0, n1;
   int e;
   normal_parts(tb, a, b, m0, m1, n0, n1, e);
-  const int s = -53 - e < 63 ? -53 - e : 63;
-  const u64 half = 1ull << (s - 1);
-  const i64 k0 = -static_cast<i64>(n0), k1 = -static_cast<i64>(n1);
-  z0 = (static_cast<i64>((m0 + half) >> s) ^ k0) - k0;
-  z1 = (static_cast<i64>((m1 + half) >> s) ^ k1) - k1;
+  z0 = normal_fx<U>(m0, n0, e);
+  z1 = normal_fx<U>(m1, n1, e);
 }
 
 // ------------------------------------------------------ Franke function ----

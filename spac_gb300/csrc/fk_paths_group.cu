@@ -5,9 +5,10 @@
 // positions are a running sum of normals that are known from the step's
 // counter alone.  The lanes of a group form G steps' normals at once, a scan
 // gives the G positions, every lane evaluates the source and the exit test at
-// its own step, and the first step that stops ends the path.  The same normals
-// and the same sums as one lane stepping G times, in another order of FP64
-// additions.
+// its own step, and the first step that stops ends the path.  The sums are those
+// of one lane stepping G times, in another order: a round's normals are added
+// in 2^-55 units (an error of 2^-56 each, times sigma sqrt(h), below the last
+// digit of a position of order 1), and the source terms by lane.
 //
 // What bounds it: in the lane-per-path kernel a call cannot end before its
 // longest path has run step by step, 1.4 us each for a warp on its own, while
@@ -92,10 +93,13 @@ __global__ void __launch_bounds__(256, 2) paths_group_kernel(const LaunchArgs a)
         const int n = k + gl;
         const uint4 r = philox10_rk(make_uint4(static_cast<uint32_t>(n), ch.p0 + pl, static_cast<uint32_t>(ch.item), a.stream),
                                     a.rkey);
-        // (the normals' running sums as integers, 2^-53 units: exact, and off the FP64 pipe)
-        fx::i64 z0, z1;
-        fx::normal_pair_fx(bvp.tab, r.x, r.y, z0, z1);
-        fx::i64 zx = z0, zy = z1;
+        // (the normals' running sums as integers, 2^-55 units: 32 normals stay below
+        // 2^63, the sums are exact and off the FP64 pipe)
+        fx::u64 m0, m1;
+        fx::u32 n0, n1;
+        int ez;
+        fx::normal_parts(bvp.tab, r.x, r.y, m0, m1, n0, n1, ez);
+        fx::i64 zx = fx::normal_fx<55>(m0, n0, ez), zy = fx::normal_fx<55>(m1, n1, ez);
 #pragma unroll
         for (int o = 1; o < G; o <<= 1) {
           const fx::i64 ux = __shfl_up_sync(kFull, zx, o, G), uy = __shfl_up_sync(kFull, zy, o, G);
@@ -104,7 +108,7 @@ __global__ void __launch_bounds__(256, 2) paths_group_kernel(const LaunchArgs a)
             zy += uy;
           }
         }
-        const R x = xs + sh * fx::to_double(zx, -53), y = ys + sh * fx::to_double(zy, -53);
+        const R x = xs + sh * fx::to_double(zx, -55), y = ys + sh * fx::to_double(zy, -55);
         R xp = __shfl_up_sync(kFull, x, 1, G), yp = __shfl_up_sync(kFull, y, 1, G);  // the step's start point
         if (gl == 0) {
           xp = xs;
@@ -120,7 +124,8 @@ __global__ void __launch_bounds__(256, 2) paths_group_kernel(const LaunchArgs a)
           const R Yn = TraitsOf<PROB>::no_potential ? R(1) : Y * pw;
           Z += TraitsOf<PROB>::no_potential ? co.f * h : (co.f * Yn) * h;
           if (cv) {
-            const R F = co.Fx * (sqrth * fx::to_double(z0, -53)) + co.Fy * (sqrth * fx::to_double(z1, -53));
+            // (the normals with all their digits: the term is as exact as they are)
+            const R F = co.Fx * (sqrth * fx::to_double(m0, n0, ez)) + co.Fy * (sqrth * fx::to_double(m1, n1, ez));
             xi += TraitsOf<PROB>::no_potential ? F : Yn * F;
           }
         }

@@ -18,7 +18,8 @@ def _lines(tmp_path_factory, name):
 
 
 def test_normal_pair_by_radius(tmp_path_factory):
-    lines = _lines(tmp_path_factory, "fixed_normals")
+    fx, *lines = _lines(tmp_path_factory, "fixed_normals")
+    assert fx[0] == "fx" and float(fx[1]) <= 0.5  # rounded to nearest
     assert {int(w[0]) for w in lines} >= set(range(-16, 3))  # radius 2^-16 (u next to 1) to 6.8
     for w in lines:
         rms, top, rms64, top64 = map(float, w[1:])

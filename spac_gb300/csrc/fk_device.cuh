@@ -462,9 +462,13 @@ struct Problem<2> {
   __device__ __noinline__ static double a_far(double x, double y) { return coef_a(x, y); }
   template <typename R>
   __device__ static R sigma_of(R a) {
-    // (a is 1/2 to 3/2: sqrt(2a) on the integer pipes)
-    if constexpr (std::is_same<R, double>::value) return fx::aniso_sigma(fx::a_bits(a));
-    else return fsqrt(R(2) * a);
+    // (a is 1/2 to 3/2, or NaN: sqrt(2a) on the integer pipes)
+    if constexpr (std::is_same<R, double>::value) {
+      const double s = fx::aniso_sigma(fx::a_bits(a));
+      return static_cast<unsigned>(__double2hiint(a)) < 0x40000000u ? s : a;
+    } else {
+      return fsqrt(R(2) * a);
+    }
   }
   template <typename R>
   __device__ __forceinline__ static void step_of(R x, R y, R a, R s, bool cv, StepCoef<R>& o) {

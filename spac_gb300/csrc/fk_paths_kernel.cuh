@@ -617,9 +617,11 @@ struct ExitTest {
   __device__ __forceinline__ bool rect_in(R x, R y, R cx, R cy, R hx, R hy) const {
     if constexpr (k64) {
       // d < thr < 0: the larger of two negative offsets, as integers (a negative
-      // double grows as its bits fall; a non-negative or NaN offset fails)
+      // double grows as its bits fall; a non-negative offset fails).  A NaN
+      // decides as in rect_dist: the ordinate's fails, the abscissa's leaves the
+      // other offset (as an integer it is above every negative one).
       const long long ox = __double_as_longlong(fabs(x - cx) - hx), oy = __double_as_longlong(fabs(y - cy) - hy);
-      return (ox < 0 && oy < 0) && __longlong_as_double(ox < oy ? ox : oy) < thr;
+      return static_cast<unsigned>(ox >> 32) > 0x7ff00000u && oy < 0 && __longlong_as_double(ox < oy ? ox : oy) < thr;
     } else {
       // (the form of the comparisons: rect_dist of a NaN abscissa is the other offset)
       const R ox = fabs(x - cx) - hx, oy = fabs(y - cy) - hy;
@@ -628,11 +630,12 @@ struct ExitTest {
   }
   __device__ __forceinline__ bool circle_in(R x, R y, R r0, R cx, R cy) const {
     if constexpr (k64) {
-      // |x - c|, at least 5e-4, below r0 + thr
+      // |x - c|, at least 5e-4, below r0 + thr (a NaN, whose normal and with it the
+      // threshold are NaN, stops)
       const R nx = x - cx, ny = y - cy, rho = r0 + thr;
       return rho > 5e-4 && nx * nx + ny * ny < rho * rho;
     } else {
-    return circle_dist<R>(x, y, r0, cx, cy).d < thr;
+      return circle_dist<R>(x, y, r0, cx, cy).d < thr;
     }
   }
   __device__ __forceinline__ bool inside(R x, R y) const {

@@ -21,6 +21,7 @@
 // the Feynman-Kac rows).
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <utility>
 
@@ -564,7 +565,11 @@ bool disk_prepare(const std::vector<DiskHost>& in, DiskBatch& out, std::string& 
   std::map<std::pair<double, int>, long long> classes;
   std::map<int, long long> modes;
   std::map<std::pair<long long, long long>, int> ops;                          // (tables, eigenvalues) -> first disk
-  std::map<std::pair<std::pair<double, int>, std::vector<double>>, int> rings;  // (grid angle, N_c), periphery angles -> first disk
+  // N_c, grid angle, periphery angles -> first disk; by their bits, which have an
+  // order for every value (with a NaN, doubles do not, and another disk's key
+  // could pass for it)
+  std::map<std::pair<int, std::vector<unsigned long long>>, int> rings;
+  auto same_bits = [](const double* a, const double* b, size_t n) { return std::memcmp(a, b, n * sizeof(double)) == 0; };
   int last_ring = -1;
   long long inner = 0, g = 0, periph = 0;
   out.has_csr = !in.empty();
@@ -624,11 +629,15 @@ bool disk_prepare(const std::vector<DiskHost>& in, DiskBatch& out, std::string& 
     out.z_total += (np + 1) * D.zstride;
     const int me = static_cast<int>(di);
     D.op_rep = ops.emplace(std::make_pair(D.tab_off, D.mu_off), me).first->second;
-    if (last_ring >= 0 && in[last_ring].theta0 == h.theta0 && in[last_ring].n_circle == h.n_circle &&
-        in[last_ring].periph_theta == h.periph_theta) {
+    if (last_ring >= 0 && in[last_ring].n_circle == h.n_circle && in[last_ring].periph_theta.size() == h.periph_theta.size() &&
+        same_bits(&in[last_ring].theta0, &h.theta0, 1) &&
+        same_bits(in[last_ring].periph_theta.data(), h.periph_theta.data(), h.periph_theta.size())) {
       D.ring_rep = last_ring;  // (the usual case, without a search)
     } else {
-      D.ring_rep = rings.emplace(std::make_pair(std::make_pair(h.theta0, h.n_circle), h.periph_theta), me).first->second;
+      std::vector<unsigned long long> key(1 + np);
+      std::memcpy(key.data(), &h.theta0, sizeof(double));
+      std::memcpy(key.data() + 1, h.periph_theta.data(), np * sizeof(double));
+      D.ring_rep = rings.emplace(std::make_pair(h.n_circle, std::move(key)), me).first->second;
       last_ring = D.ring_rep;
     }
     D.inner_off = inner;

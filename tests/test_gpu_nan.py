@@ -61,3 +61,20 @@ def test_nan_in_a_circle_stops_at_once(fk):
     r = _solve(fk, fk.DISK, (0.6, 0.0, 0.0), [[NAN, 0.1], [0.1, 0.1]], 1e-3, 100, 50, prob=(0.0, 0.0, 0.6, 0))
     assert r["n_capped"][0] == 0 and r["mean_steps"][0] == 1 and np.isnan(r["phi"][0])
     assert np.isfinite(r["phi"][1])
+
+
+def test_nan_disk_leaves_the_others_of_its_batch(gpu, fk):
+    """A disk with a NaN grid angle, before and between sound ones of several
+    angles: each of these gets the rows that it gets alone.  (Franke: the
+    operators hold no NaN.)"""
+    b = gpu.register_bvp(fk.FRANKE)
+    disks = []
+    for i, t0 in enumerate([NAN, 0.3, 0.1, NAN, 0.2, 0.1, 0.3, 0.2]):
+        th = 2 * np.pi * np.arange(16) / 16
+        c = np.array([0.4 + 0.02 * i, 0.5])
+        disks.append(dict(cx=c[0], cy=c[1], radius=0.1, theta0=t0, n_circle=16, n_radial=11, periph_theta=th,
+                          inner_xy=np.stack([c[0] + 0.05 * np.cos([0.2, 1.3]), c[1] + 0.05 * np.sin([0.2, 1.3])], 1)))
+    for d, (G, B) in zip(disks, gpu.solve_disks_ps(b, disks)):
+        if not np.isnan(d["theta0"]):
+            (g, v), = gpu.solve_disks_ps(b, [d])
+            assert np.isfinite(g).all() and np.array_equal(G, g) and np.array_equal(B, v)

@@ -218,7 +218,9 @@ __global__ void __launch_bounds__(32 * kModeWarps) disk_modes_kernel(const DiskA
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
     }
-    const int p = bi;
+    // (lane 0's, one row for all: with a NaN in the column the lanes disagree, and
+    // one beyond the rows holds its own number)
+    const int p = __shfl_sync(0xffffffffu, bi, 0);
     const double pv = S[p * ld + col];
     if (pv == 0.0) {  // uniform over the warp: singular mode matrix
       if (lane == 0) atomicOr(&a.flags[0], 1);

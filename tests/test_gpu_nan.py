@@ -78,3 +78,19 @@ def test_nan_disk_leaves_the_others_of_its_batch(gpu, fk):
         if not np.isnan(d["theta0"]):
             (g, v), = gpu.solve_disks_ps(b, [d])
             assert np.isfinite(g).all() and np.array_equal(G, g) and np.array_equal(B, v)
+
+
+def test_nan_disk_operators_leave_the_others_of_their_batch(gpu, fk):
+    """A disk whose mode matrices hold NaN (varying c at a NaN centre): its
+    elimination stays in its rows, the other disks get theirs."""
+    b = gpu.register_bvp(fk.ANISO)
+    disks = []
+    for i, cx in enumerate([0.4, NAN, 0.5, NAN]):
+        th = 0.1 + 2 * np.pi * np.arange(16) / 16
+        c = np.array([cx, 0.5])
+        disks.append(dict(cx=c[0], cy=c[1], radius=0.1, theta0=0.1, n_circle=16, n_radial=11, periph_theta=th,
+                          inner_xy=np.stack([c[0] + 0.05 * np.cos([0.2, 1.3]), c[1] + 0.05 * np.sin([0.2, 1.3])], 1)))
+    for d, (G, B) in zip(disks, gpu.solve_disks_ps(b, disks)):
+        if not np.isnan(d["cx"]):
+            (g, v), = gpu.solve_disks_ps(b, [d])
+            assert np.isfinite(g).all() and np.array_equal(G, g) and np.array_equal(B, v)

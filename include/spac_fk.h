@@ -150,6 +150,12 @@ int fk_last_timing(const fk_ctx* ctx, double out[3]);
  * G/B scatter's work, 20 moments per window.  No reference counterpart (a
  * measurement). */
 int fk_last_windows(const fk_ctx* ctx, long long* windows);
+/* Schedule of the last solve's path launch: [0] lanes per path (8 or 32: a
+ * group steps a path in parallel), [1] 1 if warps stream from chunk to chunk
+ * undrained, [2] classes of chunks of equal constants, [3] threads per block,
+ * [4] blocks, [5] paths per chunk at most.  No reference counterpart (a
+ * measurement; results do not depend on it but for the order of sums). */
+int fk_last_schedule(const fk_ctx* ctx, int out[6]);
 
 /* ---- problem registry (BVP) ---------------------------------------------- */
 int fk_register_bvp(fk_ctx* ctx, const fk_bvp_desc* desc, int* bvp_id);

@@ -2,6 +2,7 @@
 // launch sequence path kernel -> finalize/scatter on the context stream.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -142,8 +143,9 @@ struct fk_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   double timing[3] = {0, 0, 0};
-  size_t acc_clean = 0;
-  long long last_windows = 0;  // windows formed into G rows by the last solve (fk_last_windows)  // bytes at the start of w_acc known to be zero (left so by warp-mode fused launches)
+  int schedule[6] = {0, 0, 0, 0, 0, 0};  // of the last solve (fk_last_schedule)
+  size_t acc_clean = 0;        // bytes at the start of w_acc known to be zero (left so by warp-mode fused launches)
+  long long last_windows = 0;  // windows formed into G rows by the last solve (fk_last_windows)
   std::string err;
   std::vector<fk::BvpDev> bvps;
   fk::DBuf d_bvps;
@@ -890,6 +892,8 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     a.item_G = item_G;
     a.g_sum = o.g_sum;
   }
+  const int schedule[6] = {group, mix ? 1 : 0, n_cls, block_used, grid, static_cast<int>(std::min<long long>(chunk, INT_MAX))};
+  std::copy(schedule, schedule + 6, ctx->schedule);
   FK_CUDA(cudaEventRecord(ctx->ev[0], s));
   if (!chunks.empty()) {
     if (group > 1) FK_CUDA(fk::launch_paths_group(a, bvp.problem, group, grid, block_used, s));
@@ -1073,6 +1077,12 @@ int fk_cuda_stream(const fk_ctx* ctx, void** s) { if (!ctx || !s) return FK_ERR_
 int fk_last_windows(const fk_ctx* ctx, long long* windows) {
   if (!ctx || !windows) return FK_ERR_ARG;
   *windows = ctx->last_windows;
+  return FK_OK;
+}
+
+int fk_last_schedule(const fk_ctx* ctx, int out[6]) {
+  if (!ctx || !out) return FK_ERR_ARG;
+  std::copy(ctx->schedule, ctx->schedule + 6, out);
   return FK_OK;
 }
 

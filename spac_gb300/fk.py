@@ -78,6 +78,7 @@ _SIGS = {
     "fk_cuda_stream": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "fk_last_timing": (C.c_int, [C.c_void_p, _dp]),
     "fk_last_windows": (C.c_int, [C.c_void_p, C.POINTER(C.c_longlong)]),
+    "fk_last_schedule": (C.c_int, [C.c_void_p, _ip]),
     "fk_mesh_window": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_double, _ip, _ip, _ip]),
     "fk_register_bvp": (C.c_int, [C.c_void_p, C.POINTER(BvpDesc), _ip]),
     "fk_solve_points": (C.c_int, [C.c_void_p, C.c_int, C.c_int, _dp, _up, _dp, _ip, _dp, C.c_int,
@@ -251,6 +252,12 @@ class Context:
         out = C.c_longlong()
         self.check(self.L.fk_last_windows(self.h, C.byref(out)))
         return int(out.value)
+
+    def last_schedule(self):
+        """Schedule of the last solve's path launch (fk_last_schedule)."""
+        out = (C.c_int * 6)()
+        self.check(self.L.fk_last_schedule(self.h, out))
+        return dict(zip(("lanes", "streaming", "classes", "block", "grid", "chunk"), out))
 
     def last_timing(self):
         out = (C.c_double * 3)()

@@ -127,8 +127,10 @@ const char* fk_last_error(const fk_ctx* ctx);
 int fk_set_stream(fk_ctx* ctx, unsigned stream_id);
 int fk_get_stream(const fk_ctx* ctx, unsigned* stream_id);
 int fk_set_max_steps(fk_ctx* ctx, int max_steps);
-/* Launch shape of the path kernel: threads per block and paths per work
- * chunk (0 = autotuned / default). */
+/* Launch shape of the path kernel: threads per block (32..256) and paths per
+ * work chunk, 0 for the default: a shape by the call's size.  A block set here
+ * is kept, whichever kernel the call's size picks (adaptive rounds and FP64
+ * patches of thousands of nodes excepted, whose shared memory sets it). */
 int fk_set_launch(fk_ctx* ctx, int block_threads, int chunk_paths);
 /* Limits of the kernels' bounded waits, in seconds (0 restores the default).
  * slot_wait_s: a path-kernel warp's wait for a chunk slot that another warp

@@ -138,7 +138,8 @@ struct fk_ctx {
   unsigned stream_id = 0;
   int max_steps = 1 << 24;
   unsigned long long slot_wait_ns = 0, barrier_ns = 0;  // fk_set_wait_limits (0: defaults)
-  int block = 256, chunk = 0;
+  int block = 256, chunk = 0;  // launch shape (fk_set_launch)
+  bool block_set = false;      // the caller's block, to be kept (not the default)
   int num_sms = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -689,9 +690,11 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   if (group > 1) {
     // as many warps per SM as there are paths for, up to 16 (two CTAs)
     const long long want = (total_paths * group + 32LL * ctx->num_sms - 1) / (32LL * ctx->num_sms);
-    block_used = static_cast<int>(32 * std::max<long long>(1, std::min<long long>(8, want)));
-    grid = ctx->num_sms * (want > 8 ? 2 : 1);
-  } else if (mix && ctx->chunk <= 0 && lblock == 256) {
+    if (!ctx->block_set) block_used = static_cast<int>(32 * std::max<long long>(1, std::min<long long>(8, want)));
+    const int wpb = block_used / 32;  // (the caller's block: as many of them, but no more than 4, whose tables fill an SM)
+    const long long ctas = std::min<long long>((want + wpb - 1) / wpb, std::min(4, std::max(2, 16 / wpb)));
+    grid = ctx->num_sms * static_cast<int>(std::max<long long>(1, ctas));
+  } else if (mix && ctx->chunk <= 0 && !ctx->block_set && lblock == 256) {
     // Streaming: full occupancy from 4 paths per lane on; with fewer paths
     // fewer warps, whose lanes stay busy longer, but one per scheduler at
     // least (37 anisotropic points x 1,501 paths: 4.0 ms on 4 warps per SM, 4.7
@@ -1070,6 +1073,7 @@ int fk_set_launch(fk_ctx* ctx, int block, int chunk) {
   if (block != 0 && (block < 32 || block > 256 || block % 32)) return fail(ctx, FK_ERR_ARG, "block must be 32..256, multiple of 32");
   if (chunk < 0) return fail(ctx, FK_ERR_ARG, "chunk must be >= 0");
   ctx->block = block ? block : 256;
+  ctx->block_set = block != 0;
   ctx->chunk = chunk;
   return FK_OK;
 }
@@ -1262,6 +1266,7 @@ int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy,
       if (t < best) { best = t; bb = b; bc = c; }
     }
   ctx->block = bb;
+  ctx->block_set = true;
   ctx->chunk = bc;
   ctx->stream_id = saved_stream;  // tuning runs do not advance the random stream
   if (best_block) *best_block = bb;

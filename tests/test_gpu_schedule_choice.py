@@ -34,3 +34,22 @@ def test_streaming_by_paths_per_item(gpu, fk, problem, precision, paths, streami
     assert s["lanes"] == 1 and s["streaming"] == streaming and s["classes"] == 1
     gpu.solve_points(b, xy, paths, np.where(np.arange(40) % 4 == 0, 1e-3, 2e-3), getattr(fk, precision))
     assert gpu.last_schedule()["classes"] == (2 if streaming else 1)
+
+
+@pytest.mark.parametrize("block", [32, 64, 128, 256])
+@pytest.mark.parametrize("n,h,lanes", [(1001, 1e-3, 32), (100003, 4e-3, 8), (1000000, 1e-2, 1)])
+def test_callers_block_is_kept(gpu, fk, block, n, h, lanes):
+    """Whichever kernel runs, and with the default's results."""
+    b = gpu.register_bvp(fk.FRANKE)
+    out = []
+    for shape in (0, block):
+        gpu.set_launch(shape, 0)
+        gpu.set_stream(172)
+        out.append(gpu.solve_points(b, np.array([[0.45, 0.55]]), n, h, fk.FP64))
+        s = gpu.last_schedule()
+        gpu.set_launch(0, 0)
+        assert s["lanes"] == lanes
+    assert s["block"] == block and s["grid"] > 0
+    assert out[1]["n_paths"][0] == n
+    for k in out[0]:
+        assert np.allclose(out[0][k], out[1][k], rtol=1e-11, atol=1e-13), k

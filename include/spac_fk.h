@@ -130,7 +130,10 @@ int fk_set_max_steps(fk_ctx* ctx, int max_steps);
 /* Launch shape of the path kernel: threads per block (32..256) and paths per
  * work chunk, 0 for the default: a shape by the call's size.  A block set here
  * is kept, whichever kernel the call's size picks (adaptive rounds and FP64
- * patches of thousands of nodes excepted, whose shared memory sets it). */
+ * patches of thousands of nodes excepted, whose shared memory sets it).  A
+ * chunk set here is shared by the warps of a block: with a stencil they take
+ * its paths together, in a point solve each warp takes its part
+ * (chunk_paths / warps) as a chunk of its own, a lane per path. */
 int fk_set_launch(fk_ctx* ctx, int block_threads, int chunk_paths);
 /* Limits of the kernels' bounded waits, in seconds (0 restores the default).
  * slot_wait_s: a path-kernel warp's wait for a chunk slot that another warp
@@ -172,16 +175,20 @@ int fk_solve_points(fk_ctx* ctx, int bvp_id, int n, const double* xy, const unsi
 /* Batched uneven point solves: n points, each of its own registered BVP
  * (all of one problem functor and control mode), path count and step size,
  * in ONE persistent launch: chunks of every point's paths are handed to the
- * CTAs longest-first and finished paths are regenerated at once, so points
- * with 1e3 and 1e5 paths and different h share the grid without idling.
+ * warps as they run out of work and finished paths are regenerated at once,
+ * so points with 1e3 and 1e5 paths and different h share the grid without
+ * idling.  (Chunks that warps drain one by one, of FP32 points of up to 3,072
+ * paths each on average, are handed out longest-first; warps that stream from
+ * chunk to chunk need no order.)
  * No reference counterpart beyond Solve_OMP_Analytic(X0,...) called per point. */
 int fk_solve_points_multi(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy, const unsigned* paths,
                           const double* h, int precision, fk_stats* out);
 /* Autotuner of the persistent launch: times the path kernel (CUDA events) on
  * the given batched solve with every path count scaled by sample_fraction,
  * for block sizes {64, 128, 256} x chunk sizes {512, 2048, 8192, 32768}, and
- * keeps the fastest pair in the context (as fk_set_launch).  The tuning runs
- * do not advance the context's random stream id. */
+ * keeps the fastest pair in the context (as fk_set_launch, but that the lanes
+ * per path stay chosen by a call's size).  The tuning runs do not advance the
+ * context's random stream id. */
 int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy, const unsigned* paths,
                        const double* h, int precision, double sample_fraction, int* best_block, int* best_chunk,
                        double* best_ms);

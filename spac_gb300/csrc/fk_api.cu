@@ -140,6 +140,7 @@ struct fk_ctx {
   unsigned long long slot_wait_ns = 0, barrier_ns = 0;  // fk_set_wait_limits (0: defaults)
   int block = 256, chunk = 0;  // launch shape (fk_set_launch)
   bool block_set = false;      // the caller's block, to be kept (not the default)
+  bool tuned = false;          // the autotuner's shape: lanes per path stay chosen by size
   int num_sms = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -474,6 +475,9 @@ struct RunOpts {
   double* g_sum = nullptr;
   double* run_stats = nullptr;
   double* item_var = nullptr;
+  // The autotuner's runs: this share of the paths of the call that is tuned for
+  // (which picks the lanes per path).
+  double sample = 1.0;
   bool defer = false;  // queue the launch and leave the stream synchronisation and the checks to finish_run
 };
 
@@ -566,7 +570,7 @@ void group_chunks(fk_ctx* ctx, const std::vector<fk::ItemDev>& it, std::vector<f
 // are the mean exit time of the item's start point over h (exact in a disk, a
 // bound from the nearer pair of sides in a rectangle); the longest of n paths
 // is ln(n) decay times of the slowest mode.
-int group_width(const fk_ctx* ctx, const std::vector<fk::ItemDev>& it) {
+int group_width(const fk_ctx* ctx, const std::vector<fk::ItemDev>& it, double sample) {
   constexpr double kLaneCost = 360, kLaneStep = 2800, kGroupCost = 420, kGroupStep = 3300;
   double paths = 0, steps = 0, longest = 0;
   for (const fk::ItemDev& x : it) {
@@ -586,8 +590,8 @@ int group_width(const fk_ctx* ctx, const std::vector<fk::ItemDev>& it) {
     const fk::BvpDev& b = ctx->bvps[x.bvp];
     shape(b.dom_shape == FK_SHAPE_CIRCLE, b.dom);
     if (x.sub_shape >= 0) shape(x.sub_shape == FK_SHAPE_CIRCLE, x.sub);
-    paths += x.paths;
-    steps += x.paths * (1.0 + t / x.h);
+    paths += x.paths / sample;
+    steps += x.paths / sample * (1.0 + t / x.h);
     longest = std::max(longest, decay / x.h);
   }
   longest *= std::log(std::max(2.0, paths));
@@ -684,8 +688,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   int block_used = lblock;
   size_t smem_used = sacc_bytes;
   int group = 1;  // lanes per path
-  if (warp_mode && ctx->chunk <= 0 && bvp.cv != FK_CV_MLP && fk::paths_group_available(bvp.problem, precision, kind))
-    group = group_width(ctx, it);
+  // (a chunk set by the caller asks for a lane per path; the autotuner's does not)
+  if (warp_mode && (ctx->chunk <= 0 || (ctx->tuned && kind == 0)) && bvp.cv != FK_CV_MLP &&
+      fk::paths_group_available(bvp.problem, precision, kind))
+    group = group_width(ctx, it, o.sample);
   const bool mix = warp_mode && group == 1 && stream;
   if (group > 1) {
     // as many warps per SM as there are paths for, up to 16 (two CTAs)
@@ -719,8 +725,17 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // (measured on the 8x8 assembly and on point solves, finer chunks cost
   // more in per-chunk work than they save in the last round).  An item is
   // split into equal chunks (no small remainder).
+  // A chunk set by the caller is what the warps of a CTA take together: a point
+  // solve, whose chunks are one warp's each, cuts it (and a point of fewer paths)
+  // into as many parts (1,024 points x 10^4 paths in FP32 at 8,192 paths per
+  // chunk: 7.1 ms, 21.0 with one warp on each); with lane groups, the
+  // autotuner's, a path counts as its lanes.
   long long chunk = ctx->chunk;
-  if (group > 1) {
+  const bool shared_chunk = kind == 0 && chunk > 0;
+  if (shared_chunk) {
+    chunk /= block_used / 32;
+    chunk = group > 1 ? std::max<long long>(32 / group, chunk / group) : std::max<long long>(std::min(ctx->chunk, 32), chunk);
+  } else if (group > 1) {
     // short chunks: a warp takes its chunk's paths 32 / group at a time.  Arc
     // items of up to 32 paths stay whole: their moments are then summed in one
     // order, and the ill-conditioned inverse gives the same row in every run.
@@ -751,7 +766,8 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   for (int i = 0; i < n; ++i) {
     if (it[i].frontera || it[i].paths == 0) continue;
     const long long np = it[i].paths;
-    const long long pieces = (np + chunk - 1) / chunk;
+    long long pieces = (np + chunk - 1) / chunk;
+    if (shared_chunk) pieces = std::max(pieces, std::min<long long>(block_used / 32, (np + 31) / 32));
     const long long per = (np + pieces - 1) / pieces;
     for (long long p0 = 0; p0 < np; p0 += per) {
       const long long p1 = std::min<long long>(np, p0 + per);
@@ -1074,6 +1090,7 @@ int fk_set_launch(fk_ctx* ctx, int block, int chunk) {
   if (chunk < 0) return fail(ctx, FK_ERR_ARG, "chunk must be >= 0");
   ctx->block = block ? block : 256;
   ctx->block_set = block != 0;
+  ctx->tuned = false;
   ctx->chunk = chunk;
   return FK_OK;
 }
@@ -1245,6 +1262,8 @@ int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy,
   const int chunks[] = {512, 2048, 8192, 32768};
   int bb = 256, bc = 0;
   double best = 1e300;
+  ctx->block_set = true;
+  ctx->tuned = true;
   for (int b : blocks)
     for (int c : chunks) {
       if (c % b) continue;
@@ -1255,6 +1274,7 @@ int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy,
         RunOut ro;
         RunOpts opts;
         opts.multi_bvp = true;
+        opts.sample = sample_fraction;
         rc = run_items(ctx, bvp_ids[0], precision, items, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, ro,
                        opts);
         if (rc && rc != FK_ERR_STEP_CAP) {
@@ -1266,7 +1286,6 @@ int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy,
       if (t < best) { best = t; bb = b; bc = c; }
     }
   ctx->block = bb;
-  ctx->block_set = true;
   ctx->chunk = bc;
   ctx->stream_id = saved_stream;  // tuning runs do not advance the random stream
   if (best_block) *best_block = bb;

@@ -53,3 +53,42 @@ def test_callers_block_is_kept(gpu, fk, block, n, h, lanes):
     assert out[1]["n_paths"][0] == n
     for k in out[0]:
         assert np.allclose(out[0][k], out[1][k], rtol=1e-11, atol=1e-13), k
+
+
+# the last: FP32, more paths than the machine has lanes for
+@pytest.mark.parametrize("problem,precision,n,paths,h", [(0, "FP64", 1, 1000, 1e-3), (0, "FP64", 64, 4000, 1e-3), (2, "FP64", 37, 1501, 1e-3),
+                                                         (3, "FP64", 5, 20000, 1e-3), (2, "FP32", 256, 10000, 1e-3)])
+def test_tuned_shape_keeps_the_lanes_of_the_size(gpu, fk, problem, precision, n, paths, h):
+    """The autotuner times shapes of the schedule that the tuned call runs: its
+    lanes per path are the untuned call's, and so are its results."""
+    dom, prob = ((0.5, 0.5, 0.5), (0.5, 0.5, 0.5, 0)) if problem == fk.DISK else ((0, 0, 1, 1), (0, 0, 0, 0))
+    b = gpu.register_bvp(problem, dom=dom, prob=prob)
+    xy = np.random.default_rng(2).uniform(0.3, 0.7, (n, 2))
+    ids, p, hh = np.full(n, b, dtype=np.int32), np.full(n, paths, dtype=np.uint32), np.full(n, h)
+    prec = getattr(fk, precision)
+    out = []
+    for tune in (False, True):
+        gpu.set_launch(0, 0)
+        if tune:
+            block, chunk, _ = gpu.autotune_points(ids, xy, p, hh, prec, sample_fraction=0.25)
+        gpu.set_stream(173)
+        out.append((gpu.solve_points_multi(ids, xy, p, hh, prec), gpu.last_schedule()))
+    gpu.set_launch(0, 0)
+    s = out[1][1]
+    assert s["lanes"] == out[0][1]["lanes"] and s["block"] == block
+    assert s["chunk"] == max(32, chunk // (block // 32)) // s["lanes"]  # the warps of a block share a chunk, a path counts as its lanes
+    tol = 1e-11 if precision == "FP64" else 1e-6
+    for k in out[0][0]:
+        assert np.allclose(out[0][0][k], out[1][0][k], rtol=tol, atol=tol), k
+
+
+@pytest.mark.parametrize("shape", [(256, 8192), (64, 8192), (256, 40), (32, 7)])
+def test_callers_chunk_is_the_blocks(gpu, fk, shape):
+    """A point solve's warps take the caller's chunk in parts, a lane per path."""
+    b = gpu.register_bvp(fk.FRANKE)
+    gpu.set_launch(*shape)
+    st = gpu.solve_points(b, np.array([[0.4, 0.5], [0.6, 0.6]]), 5000, 1e-3, fk.FP64)
+    s = gpu.last_schedule()
+    gpu.set_launch(0, 0)
+    assert s["lanes"] == 1 and s["chunk"] == max(min(shape[1], 32), shape[1] // (shape[0] // 32))
+    assert (st["n_paths"] == 5000).all()

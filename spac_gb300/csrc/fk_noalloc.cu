@@ -114,17 +114,25 @@ cudaError_t scratch_address(int dev, unsigned char** out) {
 
 // One CTA of kPrepThreads threads writes the BVP record, one item per point
 // and the work chunks: every point's paths in equal chunks of at most `chunk`
-// paths (as fk_solve_points splits them), where `chunk` is about a quarter of
-// the paths per CTA of the grid, 256..32768, and large enough that the chunk
-// count stays within kNoAllocMaxChunks.  Thread t covers points
-// [t*per, (t+1)*per): their chunk counts are scanned across the CTA.
+// paths.  The launch streams and a chunk is one warp's, as in fk_solve_points:
+// `chunk` is a warp's share of the paths over `slices` (32 in FP64, 8 in FP32),
+// min_chunk..512, and large enough that the chunk count stays within
+// kNoAllocMaxChunks.  With chunks for 8-warp CTAs (a quarter of the paths per
+// CTA, 256..32768) half the warps had none: one point x 4e6 paths in FP32 9.9
+// ms, 1,024 points x 10^4 17.1, here 3.1 and 6.4.  FP64 paths, whose steps
+// are long chains, spread over more warps from 32 paths a chunk on; FP32 takes
+// 64 once there are 32 for every warp (one point x 2e5 paths: 0.57 ms, 0.68 in chunks of 32).
+// Thread t covers points [t*per, (t+1)*per): their chunk counts are scanned
+// across the CTA; a point of many chunks is listed by all threads.
 __global__ void __launch_bounds__(kPrepThreads) noalloc_prepare(BvpDev bvp, int n, const double* xy,
-                                                                const unsigned* paths, const double* h, int grid,
+                                                                const unsigned* paths, const double* h, int warps, int slices,
                                                                 BvpDev* d_bvp, ItemDev* items, ChunkDev* chunks,
                                                                 int* n_chunks) {
   __shared__ unsigned long long s_total[kPrepThreads / 32];
   __shared__ int s_cnt[kPrepThreads / 32];
   __shared__ long long s_chunk;
+  constexpr int kMany = 256;  // chunks of a point that all threads list
+  __shared__ int s_many[kNoAllocMaxChunks / kMany], s_base[kNoAllocMaxChunks / kMany], s_n_many;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int per = (n + kPrepThreads - 1) / kPrepThreads;
   const int i0 = min(n, t * per), i1 = min(n, i0 + per);
@@ -136,12 +144,14 @@ __global__ void __launch_bounds__(kPrepThreads) noalloc_prepare(BvpDev bvp, int 
   if (t == 0) {
     unsigned long long total = 0;
     for (int w = 0; w < kPrepThreads / 32; ++w) total += s_total[w];
-    long long c = static_cast<long long>(total / (4ull * static_cast<unsigned long long>(grid)));
-    c = c < 256 ? 256 : (c > 32768 ? 32768 : c);
+    const long long min_chunk = slices <= 8 && total > 32ull * static_cast<unsigned long long>(warps) ? 64 : 32;
+    long long c = static_cast<long long>(total / (static_cast<unsigned long long>(slices) * static_cast<unsigned long long>(warps)));
+    c = c < min_chunk ? min_chunk : (c > 512 ? 512 : c);
     // each point gives at most paths/chunk + 1 chunks
     const long long room = kNoAllocMaxChunks - n;
     const long long need = static_cast<long long>((total + room - 1) / room);
     s_chunk = c > need ? c : need;
+    s_n_many = 0;
     *d_bvp = bvp;
   }
   __syncthreads();
@@ -192,9 +202,26 @@ __global__ void __launch_bounds__(kPrepThreads) noalloc_prepare(BvpDev bvp, int 
     if (np == 0) continue;
     const long long pieces = (np + chunk - 1) / chunk;
     const long long each = (np + pieces - 1) / pieces;
+    const int n_ch = static_cast<int>((np + each - 1) / each);
+    if (n_ch > kMany) {
+      const int k = atomicAdd(&s_n_many, 1);
+      s_many[k] = i;
+      s_base[k] = base;
+      base += n_ch;
+      continue;
+    }
     for (long long p0 = 0; p0 < np; p0 += each) {
       const long long p1 = p0 + each < np ? p0 + each : np;
       chunks[base++] = ChunkDev{i, static_cast<unsigned>(p0), static_cast<unsigned>(p1)};
+    }
+  }
+  __syncthreads();
+  for (int k = 0; k < s_n_many; ++k) {
+    const int i = s_many[k];
+    const long long np = paths[i], pieces = (np + chunk - 1) / chunk, each = (np + pieces - 1) / pieces;
+    for (long long c = t; c * each < np; c += kPrepThreads) {
+      const long long p0 = c * each, p1 = p0 + each < np ? p0 + each : np;
+      chunks[s_base[k] + c] = ChunkDev{i, static_cast<unsigned>(p0), static_cast<unsigned>(p1)};
     }
   }
 }
@@ -247,7 +274,7 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   // the work counter, the status words and the FP64 sums start at zero on every call
   if (cudaMemsetAsync(d_queue, 0, 4 * sizeof(int), s) != cudaSuccess) return FK_ERR_CUDA;
   if (cudaMemsetAsync(d_stats, 0, sizeof(double) * kNumStats * n, s) != cudaSuccess) return FK_ERR_CUDA;
-  noalloc_prepare<<<1, kPrepThreads, 0, s>>>(b, n, d_xy, d_paths, d_h, grid, d_bvp, d_items, d_chunks, d_queue + 4);
+  noalloc_prepare<<<1, kPrepThreads, 0, s>>>(b, n, d_xy, d_paths, d_h, grid * (block / 32), precision == FK_FP64 ? 32 : 8, d_bvp, d_items, d_chunks, d_queue + 4);
   if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
 
   LaunchArgs a;

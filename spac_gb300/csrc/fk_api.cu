@@ -631,7 +631,7 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // one pass over the items: accumulator offsets, control variates, path
   // totals, the largest stencil and the live items
   bool any_cv = false;  // some item has a control variate: the kernel build with the xi terms
-  long long total_paths = 0, n_live = 0;
+  long long total_paths = 0, n_live = 0, max_paths = 0;
   int smem_nodes = 0;
   const int n_bvps = static_cast<int>(ctx->bvps.size());
   for (auto& x : it) {
@@ -645,7 +645,10 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
       acc_words = std::max<int>(acc_words, static_cast<int>(w));
       smem_nodes = std::max(smem_nodes, S->size_of(x.stencil));
     }
-    if (!x.frontera) total_paths += x.paths;
+    if (!x.frontera) {
+      total_paths += x.paths;
+      max_paths = std::max<long long>(max_paths, x.paths);
+    }
     if (!x.frontera && x.paths > 0) ++n_live;
   }
   // chunks: balance the persistent grid
@@ -692,7 +695,13 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   if (warp_mode && (ctx->chunk <= 0 || (ctx->tuned && kind == 0)) && bvp.cv != FK_CV_MLP &&
       fk::paths_group_available(bvp.problem, precision, kind))
     group = group_width(ctx, it, o.sample);
-  const bool mix = warp_mode && group == 1 && stream;
+  // Arc items of up to 64 paths, which no rule splits into chunks of different
+  // warps (or, with lane groups, into more than two), are not streamed: a row's
+  // moments are then summed in one order, and the ill-conditioned inverse gives
+  // the same row in every run.  Streaming mixes the items in its batches of
+  // exits: 1e-7 of the largest entry between runs on 4 x 4 circles of 44 nodes,
+  // for 1.66 ms in place of 1.81 (20 paths an item, anisotropic).
+  const bool mix = warp_mode && group == 1 && stream && !(kind == 1 && max_paths <= 64);
   if (group > 1) {
     // as many warps per SM as there are paths for, up to 16 (two CTAs)
     const long long want = (total_paths * group + 32LL * ctx->num_sms - 1) / (32LL * ctx->num_sms);
@@ -736,9 +745,8 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     chunk /= block_used / 32;
     chunk = group > 1 ? std::max<long long>(32 / group, chunk / group) : std::max<long long>(std::min(ctx->chunk, 32), chunk);
   } else if (group > 1) {
-    // short chunks: a warp takes its chunk's paths 32 / group at a time.  Arc
-    // items of up to 32 paths stay whole: their moments are then summed in one
-    // order, and the ill-conditioned inverse gives the same row in every run.
+    // short chunks: a warp takes its chunk's paths 32 / group at a time; arc items
+    // of up to 64 paths in two parts at most, whose sum has one order
     const long long ng = 32 / group;
     chunk = total_paths / (2LL * grid * (block_used / 32));
     chunk = std::max<long long>(std::max<long long>(kind == 1 ? 32 : ng, total_paths >> 20), std::min(chunk, 32 * ng));

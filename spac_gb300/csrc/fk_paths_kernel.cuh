@@ -591,6 +591,35 @@ __device__ __forceinline__ void dentro_exit(R x, R y, bool dom_can_win, bool has
   }
 }
 
+// The exit test for a circle smaller than the shift and 5e-4: within 5e-4 of its
+// centre the normal is (x - c) / 5e-4 and with it the shift shrinks, so that a
+// path may go on there.  Dentro's rule as it stands: the larger distance, and
+// the shift along its normal.
+template <bool ROUND_DOM>
+static __device__ __noinline__ bool inside_tiny(double x, double y, bool dom, bool sub, bool round_sub, double dcx, double dcy,
+                                                double dhx, double dhy, double scx, double scy, double shx, double shy,
+                                                double thr) {
+  double d = -1e300, len = 1.0;  // distance and the normal's length
+  auto near = [&](bool round, double cx, double cy, double hx, double hy) {
+    double e, l = 1.0;
+    if (round) {
+      const double rr = sqrt((x - cx) * (x - cx) + (y - cy) * (y - cy)), r = rr > 5e-4 ? rr : 5e-4;
+      e = r - hx;
+      l = rr / r;
+    } else {
+      const double ox = fabs(x - cx) - hx, oy = fabs(y - cy) - hy;
+      e = ox > oy ? ox : oy;
+    }
+    if (!(d >= e)) {
+      d = e;
+      len = l;
+    }
+  };
+  if (dom) near(ROUND_DOM, dcx, dcy, dhx, dhy);
+  if (sub) near(round_sub, scx, scy, shx, shy);
+  return d < thr * len;
+}
+
 // The exit test of Dentro.  A path goes on iff every boundary's signed
 // distance is below the (negative) threshold, so a step forms the distances
 // alone, from centres and half sides kept here; Dentro's choice of boundary,
@@ -628,20 +657,29 @@ struct ExitTest {
       return oy < thr && !(ox >= thr);
     }
   }
-  __device__ __forceinline__ bool circle_in(R x, R y, R r0, R cx, R cy) const {
+  // FP64: |x - c|, at least 5e-4, below r0 + thr (a NaN, whose normal and with it
+  // the threshold are NaN, stops); tiny: a circle that inside_tiny decides
+  __device__ __forceinline__ bool circle_in(R x, R y, R r0, R cx, R cy, bool& tiny) const {
     if constexpr (k64) {
-      // |x - c|, at least 5e-4, below r0 + thr (a NaN, whose normal and with it the
-      // threshold are NaN, stops)
       const R nx = x - cx, ny = y - cy, rho = r0 + thr;
-      return rho > 5e-4 && nx * nx + ny * ny < rho * rho;
+      tiny = !(rho > 5e-4);
+      return nx * nx + ny * ny < rho * rho;
     } else {
       return circle_dist<R>(x, y, r0, cx, cy).d < thr;
     }
   }
   __device__ __forceinline__ bool inside(R x, R y) const {
-    bool in = true;
-    if (dom) in = DomainOf<PROB>::shape == 1 ? circle_in(x, y, dhx, dcx, dcy) : rect_in(x, y, dcx, dcy, dhx, dhy);
-    if (sub) in = in && (circle ? circle_in(x, y, shx, scx, scy) : rect_in(x, y, scx, scy, shx, shy));
+    bool in = true, tiny = false;
+    if (sub) in = circle ? circle_in(x, y, shx, scx, scy, tiny) : rect_in(x, y, scx, scy, shx, shy);
+    if (dom) {
+      bool t = false;
+      in = in && (DomainOf<PROB>::shape == 1 ? circle_in(x, y, dhx, dcx, dcy, t) : rect_in(x, y, dcx, dcy, dhx, dhy));
+      tiny = tiny || t;
+    }
+    if constexpr (k64) {
+      if (__builtin_expect(tiny, 0))
+        in = inside_tiny<DomainOf<PROB>::shape == 1>(x, y, dom, sub, circle, dcx, dcy, dhx, dhy, scx, scy, shx, shy, thr);
+    }
     return in;
   }
 };

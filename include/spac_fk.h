@@ -138,7 +138,9 @@ int fk_set_launch(fk_ctx* ctx, int block_threads, int chunk_paths);
 /* Limits of the kernels' bounded waits, in seconds (0 restores the default).
  * slot_wait_s: a path-kernel warp's wait for a chunk slot that another warp
  * of its CTA is still refilling (default 60 s + 1 us x max_steps, far above
- * any real wait, which the step cap bounds); barrier_s: a CTA's wait at a
+ * any real wait, which the step cap bounds; only launches with chunk slots
+ * wait: stencils of many paths per item, adaptive rounds, and stencils with a
+ * chunk set by the caller); barrier_s: a CTA's wait at a
  * grid barrier of the persistent MLP trainer (default 5 s).  A wait that runs
  * out ends its kernel early and the call returns FK_ERR_CUDA ("... timed
  * out"); the context stays usable, and that call's outputs (or the network's

@@ -13,10 +13,10 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "_build", "libfk_oracle.so")
 REF_LIB = os.path.join(HERE, "_ref", "libspac_ref.so")
-# where the reference's sources lie; a folder without them counts as absent (REF_SRC then names none)
+# where the reference's sources lie; "" without them
 REF_SRC = "/root/reference"
 if not os.path.exists(os.path.join(REF_SRC, "BVP", "BVP.hpp")):
-    REF_SRC = os.path.join(REF_SRC, "BVP")
+    REF_SRC = ""
 
 RNG_PHILOX, RNG_SEQUENTIAL = 0, 1
 RECT, CIRCLE = 0, 1

@@ -224,7 +224,8 @@ const void* select_paths_plain(int problem, int precision, int st, bool warp_mod
 // coefficients, no learned control variate
 bool paths_group_available(int problem, int precision, int stencil_kind);
 cudaError_t launch_paths_group(const LaunchArgs& a, int problem, int g, int grid, int block, cudaStream_t s);
-// stream: the streaming build of FP32 point solves
+// stream: the streaming build of point solves, of several classes (FP64 launches
+// of one class run another build with the same 2 CTAs of 256)
 int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem,
                            bool warp_mode = false, bool stream = false);
 // host launchers (fk_kernels.cu)

@@ -274,7 +274,8 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   // the work counter, the status words and the FP64 sums start at zero on every call
   if (cudaMemsetAsync(d_queue, 0, 4 * sizeof(int), s) != cudaSuccess) return FK_ERR_CUDA;
   if (cudaMemsetAsync(d_stats, 0, sizeof(double) * kNumStats * n, s) != cudaSuccess) return FK_ERR_CUDA;
-  noalloc_prepare<<<1, kPrepThreads, 0, s>>>(b, n, d_xy, d_paths, d_h, grid * (block / 32), precision == FK_FP64 ? 32 : 8, d_bvp, d_items, d_chunks, d_queue + 4);
+  noalloc_prepare<<<1, kPrepThreads, 0, s>>>(b, n, d_xy, d_paths, d_h, grid * (block / 32), precision == FK_FP64 ? 32 : 8,
+                                             d_bvp, d_items, d_chunks, d_queue + 4);
   if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
 
   LaunchArgs a;

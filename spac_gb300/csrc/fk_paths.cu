@@ -43,7 +43,8 @@ size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block, size_t smem,
                          cudaStream_t s, bool warp_mode) {
   if (block < 32 || block > 256 || block % 32 != 0) return cudaErrorInvalidValue;
-  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0, a.mix && (precision == 1 || a.n_cls > 1));
+  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0,
+                                a.mix && (precision == 1 || a.n_cls > 1));
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<LaunchArgs*>(&a)};

@@ -17,9 +17,10 @@
 // point solves of many paths stream from chunk to chunk (see paths_kernel).
 //
 // An exiting lane only pushes its exit (X_tau, or the point it stopped at
-// where the projection follows later, Y, Z, xi, steps, flags) onto its warp's shared-memory queue and starts the next path; once 32 exits are
-// queued the whole warp processes them, one exit per lane, so the exit work
-// runs at full SIMD width:
+// where the projection follows later, Y, Z, xi, steps, flags) onto its warp's
+// shared-memory queue and starts the next path; once 32 exits are queued the
+// whole warp processes them, one exit per lane, so the exit work runs at full
+// SIMD width:
 //  - exit value u(X_tau), B and the statistics into per-thread registers
 //    (compensated FP32 sums for FP32 stepping, FP64 for FP64 stepping);
 //  - the stencil moments Y phi of subdomain exits into the chunk's
@@ -1379,79 +1380,79 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
           ex = x;  // (Dentro's boundary follows when the queued exits are processed)
           ey = y;
         } else {
-        Bnd<R> w;
-        if (dom_can_win) {
-          w = (DomainOf<PROB>::shape == 1) ? circle_dist<R>(x, y, d0, d1, d2) : rect_dist<R>(x, y, d0, d1, d2, d3);
-          if (has_sub) {
-            const Bnd<R> sb = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
-            if (!(w.d >= sb.d)) { w = sb; dom_wins = false; }
-          }
-        } else {
-          w = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
-          dom_wins = false;
-        }
-        // sigma at the new point (kept for the next step) or at the
-        // projection: one evaluation at the selected point, no divergence
-        const bool inside = w.d < R(0);
-        const R stq = Problem<PROB>::template state<R>(bvp, inside ? x : w.ex, inside ? y : w.ey);
-        const R sg = Problem<PROB>::template sigma_of<R>(stq);
-        if (inside) {
-          st = stq;
-          sgc = sg;
-        }
-        // Gobet shift kGobet |sigma^T n| sqrt(h) (FeynmanKacSolver.cpp:85,92).
-        // Every registered sigma is s I, and the normals are unit vectors (axes
-        // or the normalised diagonal), so FP32 stepping takes |sigma^T n| = s;
-        // FP64 stepping forms the norm as the reference does.
-        R thr;
-        if constexpr (std::is_same<R, float>::value) {
-          thr = R(kGobet) * sg * sqrth;
-        } else {
-          const R nsx = w.nx * sg, nsy = w.ny * sg;
-          thr = R(kGobet) * fsqrt(nsx * nsx + nsy * nsy) * sqrth;
-        }
-        capped = k >= a.max_steps;
-        exits = !(w.d < thr) || capped;
-        if constexpr (RobinOf<PROB>::value) {
-          if (rmask && dom_wins && robin_side<R>(w, rmask) >= 0) {
-            // The nearest boundary is a reflecting side: no stop there
-            // (dentro / reflejada, :82-84).  The path still stops within the
-            // Gobet band of the subdomain or of an absorbing side, the
-            // nearer of them (the reference tests only the nearest boundary,
-            // which lets paths near a mixed corner cross the absorbing side).
-            const R dref = w.d;  // the reflecting side's distance
-            R da = R(-FLT_MAX);
-            int qa = -1;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if ((rmask >> q) & 1) continue;
-              const R dq = q == 0 ? d0 - x : (q == 1 ? d1 - y : (q == 2 ? x - d2 : y - d3));
-              if (dq > da) { da = dq; qa = q; }
-            }
-            if (qa >= 0) {
-              w.d = da;
-              w.ex = qa == 0 ? d0 : (qa == 2 ? d2 : fmin(fmax(x, d0), d2));
-              w.ey = qa == 1 ? d1 : (qa == 3 ? d3 : fmin(fmax(y, d1), d3));
-            } else {
-              w.d = R(-FLT_MAX);
-            }
+          Bnd<R> w;
+          if (dom_can_win) {
+            w = (DomainOf<PROB>::shape == 1) ? circle_dist<R>(x, y, d0, d1, d2) : rect_dist<R>(x, y, d0, d1, d2, d3);
             if (has_sub) {
-              // (a subdomain boundary that coincides with the reflecting side,
-              // a tie that the domain wins, is not a candidate)
               const Bnd<R> sb = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
-              if (sb.d < dref && !(w.d >= sb.d)) { w = sb; dom_wins = false; }
+              if (!(w.d >= sb.d)) { w = sb; dom_wins = false; }
             }
-            exits = !(w.d < thr) || capped;
+          } else {
+            w = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
+            dom_wins = false;
           }
-          // a path that goes on from a point on (or, by rounding, just past)
-          // a reflecting side steps with sigma at that point
-          if (!exits && !inside) {
-            st = Problem<PROB>::template state<R>(bvp, x, y);
-            sgc = Problem<PROB>::template sigma_of<R>(st);
+          // sigma at the new point (kept for the next step) or at the
+          // projection: one evaluation at the selected point, no divergence
+          const bool inside = w.d < R(0);
+          const R stq = Problem<PROB>::template state<R>(bvp, inside ? x : w.ex, inside ? y : w.ey);
+          const R sg = Problem<PROB>::template sigma_of<R>(stq);
+          if (inside) {
+            st = stq;
+            sgc = sg;
           }
-        }
-        ex = w.ex;
-        ey = w.ey;
+          // Gobet shift kGobet |sigma^T n| sqrt(h) (FeynmanKacSolver.cpp:85,92).
+          // Every registered sigma is s I, and the normals are unit vectors (axes
+          // or the normalised diagonal), so FP32 stepping takes |sigma^T n| = s;
+          // FP64 stepping forms the norm as the reference does.
+          R thr;
+          if constexpr (std::is_same<R, float>::value) {
+            thr = R(kGobet) * sg * sqrth;
+          } else {
+            const R nsx = w.nx * sg, nsy = w.ny * sg;
+            thr = R(kGobet) * fsqrt(nsx * nsx + nsy * nsy) * sqrth;
+          }
+          capped = k >= a.max_steps;
+          exits = !(w.d < thr) || capped;
+          if constexpr (RobinOf<PROB>::value) {
+            if (rmask && dom_wins && robin_side<R>(w, rmask) >= 0) {
+              // The nearest boundary is a reflecting side: no stop there
+              // (dentro / reflejada, :82-84).  The path still stops within the
+              // Gobet band of the subdomain or of an absorbing side, the
+              // nearer of them (the reference tests only the nearest boundary,
+              // which lets paths near a mixed corner cross the absorbing side).
+              const R dref = w.d;  // the reflecting side's distance
+              R da = R(-FLT_MAX);
+              int qa = -1;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                if ((rmask >> q) & 1) continue;
+                const R dq = q == 0 ? d0 - x : (q == 1 ? d1 - y : (q == 2 ? x - d2 : y - d3));
+                if (dq > da) { da = dq; qa = q; }
+              }
+              if (qa >= 0) {
+                w.d = da;
+                w.ex = qa == 0 ? d0 : (qa == 2 ? d2 : fmin(fmax(x, d0), d2));
+                w.ey = qa == 1 ? d1 : (qa == 3 ? d3 : fmin(fmax(y, d1), d3));
+              } else {
+                w.d = R(-FLT_MAX);
+              }
+              if (has_sub) {
+                // (a subdomain boundary that coincides with the reflecting side,
+                // a tie that the domain wins, is not a candidate)
+                const Bnd<R> sb = sub_circle ? circle_dist<R>(x, y, s0, s1, s2) : rect_dist<R>(x, y, s0, s1, s2, s3);
+                if (sb.d < dref && !(w.d >= sb.d)) { w = sb; dom_wins = false; }
+              }
+              exits = !(w.d < thr) || capped;
+            }
+            // a path that goes on from a point on (or, by rounding, just past)
+            // a reflecting side steps with sigma at that point
+            if (!exits && !inside) {
+              st = Problem<PROB>::template state<R>(bvp, x, y);
+              sgc = Problem<PROB>::template sigma_of<R>(st);
+            }
+          }
+          ex = w.ex;
+          ey = w.ey;
         }
       }
       // ---- queue the exits; the exiting lanes start their next path at once

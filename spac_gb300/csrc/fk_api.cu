@@ -818,8 +818,11 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   const int n_cls = std::max(1, static_cast<int>(first.size()) - 1);
   FK_CUDA(fk::upload_pinned(ctx->w_items, ctx->h_items, it, s));
   FK_CUDA(fk::upload_pinned(ctx->w_chunks, ctx->h_chunks, chunks, s));
-  FK_CUDA(ctx->w_stats.ensure(std::max<size_t>(static_cast<size_t>(n) * fk::kNumStats * sizeof(double), 16)));
-  FK_CUDA(cudaMemsetAsync(ctx->w_stats.p, 0, static_cast<size_t>(n) * fk::kNumStats * sizeof(double), s));
+  // the items' sums and, in FP64, their roundings behind them
+  const bool lo = precision == FK_FP64 && !round;
+  const size_t stats_bytes = static_cast<size_t>(n) * fk::kNumStats * sizeof(double);
+  FK_CUDA(ctx->w_stats.ensure(std::max<size_t>((lo ? 2 : 1) * stats_bytes, 16)));
+  FK_CUDA(cudaMemsetAsync(ctx->w_stats.p, 0, (lo ? 2 : 1) * stats_bytes, s));
   // slot mode with every item in one chunk: the chunks store their moments,
   // so the accumulators need no zeroing
   bool all_whole = true;
@@ -877,6 +880,8 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   a.queue = ctx->w_queue.as<int>();
   a.vis_count = ctx->w_queue.as<int>() + 4;
   a.stats = ctx->w_stats.as<double>();
+  a.stats_lo = lo ? a.stats + static_cast<size_t>(n) * fk::kNumStats : nullptr;
+  a.lo_stride = fk::kNumStats;
   a.acc = round ? nullptr : ctx->w_acc.as<double>();
   a.key0 = static_cast<uint32_t>(ctx->seed);
   a.key1 = static_cast<uint32_t>(ctx->seed >> 32);
@@ -977,6 +982,8 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     f.fin_k = std::max(kcommon, 0);
   }
   f.stats = a.stats;
+  f.stats_lo = a.stats_lo;
+  f.lo_stride = a.lo_stride;
   f.acc = a.acc;
   f.stencil_kind = kind;
   f.g_off = g_off ? ctx->w_goff.as<long long>() : nullptr;

@@ -125,6 +125,10 @@ struct LaunchArgs {
   int* queue;              // [0] chunk counter, [1] error word (both zeroed before launch)
   int* vis_count;          // may be null: += windows whose moments the kernel formed into G rows
   double* stats;           // n_items * kNumStats
+  // FP64 stepping: what the additions to an item's sums rounded off, at the
+  // sums' places of records of lo_stride (null: not kept)
+  double* stats_lo;
+  int lo_stride;
   double* acc;             // stencil accumulators
   uint32_t key0, key1, stream;
   uint32_t rkey[20];        // Philox round keys from (key0, key1): set_round_keys
@@ -189,6 +193,8 @@ struct FinalizeArgs {
   const float* patch_emax;
   int split_ok;
   const double* stats;
+  const double* stats_lo;   // as in LaunchArgs, may be null and may share item_stats
+  int lo_stride;
   const double* acc;
   int stencil_kind;
   const long long* g_off;   // item -> first entry in item_G

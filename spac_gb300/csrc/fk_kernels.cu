@@ -28,7 +28,10 @@ __device__ __forceinline__ void finalize_item_head(const FinalizeArgs& a, int it
                                                    double N) {
   BvpDev bvp = a.bvp[it.bvp];
   bvp.tab = fx::tables();
-  const double* S = a.stats + static_cast<long long>(item) * kNumStats;
+  double S[kNumStats];
+  for (int k = 0; k < kNumStats; ++k) S[k] = a.stats[static_cast<long long>(item) * kNumStats + k];
+  if (a.stats_lo)
+    for (int k = 0; k < kNumStats; ++k) S[k] += a.stats_lo[static_cast<long long>(item) * a.lo_stride + k];
   double Bv;
   if (it.frontera) {
     Bv = Problem<PROB>::u(bvp, it.x, it.y);  // Solve_OMP_Analytic :346-347

@@ -274,6 +274,9 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   // the work counter, the status words and the FP64 sums start at zero on every call
   if (cudaMemsetAsync(d_queue, 0, 4 * sizeof(int), s) != cudaSuccess) return FK_ERR_CUDA;
   if (cudaMemsetAsync(d_stats, 0, sizeof(double) * kNumStats * n, s) != cudaSuccess) return FK_ERR_CUDA;
+  // FP64: the sums' roundings lie in the caller's output records until the finalize launch
+  const bool lo = precision == FK_FP64;
+  if (lo && cudaMemsetAsync(d_out, 0, sizeof(fk_stats) * n, s) != cudaSuccess) return FK_ERR_CUDA;
   noalloc_prepare<<<1, kPrepThreads, 0, s>>>(b, n, d_xy, d_paths, d_h, grid * (block / 32), precision == FK_FP64 ? 32 : 8,
                                              d_bvp, d_items, d_chunks, d_queue + 4);
   if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
@@ -288,6 +291,8 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   a.n_chunks_dev = d_queue + 4;
   a.queue = d_queue;
   a.stats = d_stats;
+  a.stats_lo = lo ? reinterpret_cast<double*>(d_out) : nullptr;
+  a.lo_stride = static_cast<int>(sizeof(fk_stats) / sizeof(double));
   a.key0 = static_cast<uint32_t>(seed);
   a.key1 = static_cast<uint32_t>(seed >> 32);
   set_round_keys(a);
@@ -306,6 +311,8 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   f.items = d_items;
   f.n_items = n;
   f.stats = d_stats;
+  f.stats_lo = a.stats_lo;
+  f.lo_stride = a.lo_stride;
   f.stencil_kind = 0;
   f.item_stats = reinterpret_cast<double*>(d_out);
   f.flags = d_queue + 2;

@@ -724,7 +724,8 @@ __device__ __forceinline__ void add_item_sums(const LaunchArgs& a, int item, con
       const double old = atomicAdd(&sums[k], v);
       if (a.stats_lo) {
         const double s = old + v, b = s - old, e = (old - (s - b)) + (v - b);
-        if (e != 0.0) atomicAdd(&a.stats_lo[static_cast<long long>(item) * a.lo_stride + k], e);
+        // (NaN where the sum is not finite, which then stays as it is)
+        if (fabs(e) > 0.0) atomicAdd(&a.stats_lo[static_cast<long long>(item) * a.lo_stride + k], e);
       }
     }
   } else {

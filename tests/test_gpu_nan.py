@@ -63,6 +63,15 @@ def test_nan_in_a_circle_stops_at_once(fk):
     assert np.isfinite(r["phi"][1])
 
 
+@pytest.mark.parametrize("n", [1, 200, 5000])
+def test_a_sum_that_overflows_is_infinite(fk, n):
+    """A start point so far below the square that the source is 1e301 per step:
+    the mean is finite, the mean square overflows and says so."""
+    r = _solve(fk, fk.FRANKE, (0, 0, 1, 1), [[0.5, -780.0], [0.5, 0.5]], 1e-3, n, 100000)
+    assert np.isfinite(r["phi"][0]) and abs(r["phi"][0]) > 1e290
+    assert np.isposinf(r["phiphi"][0]) and np.isfinite(r["phiphi"][1])
+
+
 def test_nan_disk_leaves_the_others_of_its_batch(gpu, fk):
     """A disk with a NaN grid angle, before and between sound ones of several
     angles: each of these gets the rows that it gets alone.  (Franke: the

@@ -744,12 +744,15 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   // solve, whose chunks are one warp's each, cuts it (and a point of fewer paths)
   // into as many parts (1,024 points x 10^4 paths in FP32 at 8,192 paths per
   // chunk: 7.1 ms, 21.0 with one warp on each); with lane groups, the
-  // autotuner's, a path counts as its lanes.
+  // autotuner's, a path counts as its lanes.  Not into more than 2^20 parts, as
+  // the default's chunks below (348 M paths of 16 disks at 512 a chunk: 277 ms in
+  // 5.4 M parts, 39 ms of it to list them; 246 in 1 M).
   long long chunk = ctx->chunk;
   const bool shared_chunk = kind == 0 && chunk > 0;
+  const long long least = std::max(32LL, total_paths >> 20);  // a part's paths (with lane groups: 32 lanes' worth)
   if (shared_chunk) {
-    chunk /= block_used / 32;
-    chunk = group > 1 ? std::max<long long>(32 / group, chunk / group) : std::max<long long>(std::min(ctx->chunk, 32), chunk);
+    const long long part = chunk / (block_used / 32) / group;
+    chunk = std::max(part, std::min(chunk, group > 1 ? std::max<long long>(32 / group, total_paths >> 20) : least));
   } else if (group > 1) {
     // short chunks: a warp takes its chunk's paths 32 / group at a time; arc items
     // of up to 64 paths in two parts at most, whose sum has one order
@@ -781,7 +784,7 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     if (it[i].frontera || it[i].paths == 0) continue;
     const long long np = it[i].paths;
     long long pieces = (np + chunk - 1) / chunk;
-    if (shared_chunk) pieces = std::max(pieces, std::min<long long>(block_used / 32, (np + 31) / 32));
+    if (shared_chunk) pieces = std::max(pieces, std::min(block_used / 32LL, (np + least - 1) / least));
     const long long per = (np + pieces - 1) / pieces;
     for (long long p0 = 0; p0 < np; p0 += per) {
       const long long p1 = std::min<long long>(np, p0 + per);

@@ -127,3 +127,16 @@ def test_fp64_sums_do_not_depend_on_their_parts(gpu, fk):
     gpu.set_launch(0, 0)
     d = (out[0] - out[1]) / out[0]
     assert np.sqrt(np.mean(d * d)) <= 2.0 ** -52, np.sqrt(np.mean(d * d)) * 2.0 ** 53
+
+
+@pytest.mark.parametrize("paths,block,chunk,part", [(1 << 20, 256, 8192, 1024), (1 << 20, 256, 512, 64), (1 << 20, 32, 16, 16),
+                                                    (100_000_000, 256, 512, 95), (100_000_000, 256, 8192, 1024)])
+def test_parts_of_a_callers_chunk(gpu, fk, paths, block, chunk, part):
+    """A warp takes its part of the caller's chunk, but the host lists no more than
+    2^20 parts for it (100 M paths >> 20 = 95)."""
+    b = gpu.register_bvp(fk.FRANKE)
+    gpu.set_launch(block, chunk)
+    st = gpu.solve_points(b, np.array([[0.05, 0.05]]), paths, 1e-2, fk.FP32)
+    s = gpu.last_schedule()
+    gpu.set_launch(0, 0)
+    assert s["chunk"] == part and s["block"] == block and st["n_paths"][0] == paths

@@ -217,7 +217,9 @@ int fk_autotune_points(fk_ctx* ctx, int n, const int* bvp_ids, const double* xy,
  * Errors found by the kernels are not returned (the call does not wait for
  * them): a point solved completely has d_out[i].n_paths == d_paths[i] and
  * d_out[i].n_capped == 0; a smaller n_paths means the kernel gave up on some
- * of the point's paths, and n_capped counts paths stopped at max_steps. */
+ * of the point's paths, and n_capped counts paths stopped at max_steps.  In
+ * FP64 the call clears d_out when it starts and keeps partial sums in it until
+ * the point is complete; n_paths and n_capped are 0 until then. */
 #define FK_NOALLOC_MAX_POINTS 16384
 int fk_solve_points_noalloc(const fk_bvp_desc* bvp, unsigned long long seed, unsigned stream_id, int n,
                             const double* d_xy, const unsigned* d_paths, const double* d_h, int precision,

@@ -29,6 +29,7 @@
 #include <cuda.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 
@@ -50,6 +51,14 @@ constexpr size_t kChunksOff = align256(kItemsOff + sizeof(ItemDev) * FK_NOALLOC_
 constexpr size_t kStatsOff = align256(kChunksOff + sizeof(ChunkDev) * kNoAllocMaxChunks);
 constexpr size_t kEnd = kStatsOff + sizeof(double) * kNumStats * FK_NOALLOC_MAX_POINTS;
 static_assert(kEnd <= kNoAllocBytes, "no-alloc scratch layout exceeds the reserved array");
+// The FP64 sums' roundings within an output record: n_paths, by which a caller
+// sees that a point is complete, then lies where the steps' would, and n_capped
+// where the domain exits' would, and counts are exact.
+constexpr int kLoOff = 4;
+static_assert(kLoOff + kNumStats <= static_cast<int>(sizeof(fk_stats) / sizeof(double)) &&
+                  offsetof(fk_stats, n_paths) == sizeof(double) * (kLoOff + kStatSteps) &&
+                  offsetof(fk_stats, n_capped) == sizeof(double) * (kLoOff + kStatDom),
+              "the roundings lie beside the completion counts");
 static_assert(sizeof(BvpDev) <= kQueueOff - kBvpOff, "BVP record does not fit its slot");
 static_assert(FK_NOALLOC_MAX_POINTS <= 16 * kPrepThreads, "prepare kernel covers at most 16 points per thread");
 
@@ -291,7 +300,7 @@ extern "C" int fk_solve_points_noalloc(const fk_bvp_desc* d, unsigned long long 
   a.n_chunks_dev = d_queue + 4;
   a.queue = d_queue;
   a.stats = d_stats;
-  a.stats_lo = lo ? reinterpret_cast<double*>(d_out) : nullptr;
+  a.stats_lo = lo ? reinterpret_cast<double*>(d_out) + kLoOff : nullptr;
   a.lo_stride = static_cast<int>(sizeof(fk_stats) / sizeof(double));
   a.key0 = static_cast<uint32_t>(seed);
   a.key1 = static_cast<uint32_t>(seed >> 32);

@@ -761,14 +761,12 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
     chunk = std::max<long long>(std::max<long long>(kind == 1 ? 32 : ng, total_paths >> 20), std::min(chunk, 32 * ng));
   } else if (mix && chunk <= 0) {
     // Streaming: 64 to 512 paths, about 32 chunks per warp for point solves
-    // (1,024 points x 10^4 paths in FP64: 14.9 ms at 64 paths, 15.0 at 128,
-    // 16.7 at 512; 16 uneven disks in FP32: 46.1 at 128, 48.2 at 512, but the
-    // host lists every chunk, 8 ms for 88 M paths in pieces of 128), 8 with
-    // a stencil (8x8 FP64 assembly: 15.6 ms at 512,
-    // 15.9 at 128) and 8 in FP32, whose kernels are five times shorter for the
-    // same list (1,024 points x 10^4 paths: 3.30 ms a call with 342 paths a chunk,
-    // 4.20 with 85, 1.0 of it for the list); never
-    // more than 2^20 chunks.
+    // (1,024 points x 10^4 paths in FP64: 16.6 ms a call at 64 paths, 16.1 at 128,
+    // 16.6 at 512), 8 with a stencil (8x8 FP64 assembly, before its terms were
+    // made finer: 15.6 ms at 512, 15.9 at 128) and 8 in FP32, whose kernels are
+    // five times shorter for the same list (1,024 points x 10^4 paths: 3.29 ms a
+    // call with 342 paths a chunk, 3.61 with 85, 0.4 of it for the list; 16 uneven
+    // disks, 90 M paths: 63.6 at 512, 66.5 at 128); never more than 2^20 chunks.
     chunk = total_paths / ((kind == 0 && precision == FK_FP64 ? 32LL : 8LL) * grid * (block_used / 32));
     chunk = std::max<long long>(std::max<long long>(64, total_paths >> 20), std::min<long long>(chunk, 512));
   } else if (chunk <= 0 && warp_mode) {

@@ -687,11 +687,11 @@ int run_items(fk_ctx* ctx, int bvp_id, int precision, std::vector<fk::ItemDev>& 
   }
   if (round && warp_mode && !wms) warp_mode = false;  // (rounds need rows formed in the kernel)
   size_t sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
-  if (sacc_bytes > 200 * 1024 && warp_mode && precision == FK_FP64 && lblock > 32) {  // (room for the tables: fewer warps)
+  if (sacc_bytes > fk::kPathsSmemMax && warp_mode && precision == FK_FP64 && lblock > 32) {  // (room for the tables: fewer warps)
     lblock = std::max(32, lblock / 64 * 32);
     sacc_bytes = fk::paths_smem_bytes(precision, kind, acc_words, smem_nodes, warp_mode, lblock, wms);
   }
-  if (sacc_bytes > 200 * 1024) return fail(ctx, FK_ERR_CAPACITY, "stencil accumulators exceed shared memory");
+  if (sacc_bytes > fk::kPathsSmemMax) return fail(ctx, FK_ERR_CAPACITY, "stencil accumulators exceed shared memory");
   const int occ = fk::paths_kernel_occupancy(bvp.problem, precision, kind, any_cv ? 1 : 0, lblock, sacc_bytes, warp_mode, stream);
   int grid = std::max(1, ctx->num_sms * occ);
   int block_used = lblock;

@@ -219,6 +219,7 @@ struct FinalizeArgs {
 // the items' global accumulators (items of few paths); otherwise the CTA's
 // warps share chunk slots with shared-memory accumulators
 // wm_shared: warp mode with per-warp FP32 moment accumulators in shared memory
+constexpr size_t kPathsSmemMax = 200 * 1024;  // dynamic shared memory of a path kernel's CTA at most
 size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem_nodes, bool warp_mode = false,
                         int block = 256, bool wm_shared = false);
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block,

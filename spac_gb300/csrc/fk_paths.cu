@@ -18,7 +18,7 @@ const void* select_paths_v(int problem, int precision, int st, bool warp_mode, b
 }
 // The variant a launch uses: the 4-CTA build for FP32 patch-stencil slot
 // mode when 4 of its CTAs fit on an SM with this shared memory and block.
-const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv, bool mode2) {
+const void* select_paths(int problem, int precision, int st, bool warp_mode, int block, size_t smem, bool cv, bool alt) {
   if (precision == 1 && st == 2 && !warp_mode && block == 256) {
     const void* f4 = select_paths_v(problem, precision, st, warp_mode, true, cv);
     int n = 0;
@@ -27,24 +27,32 @@ const void* select_paths(int problem, int precision, int st, bool warp_mode, int
       return f4;
     cudaGetLastError();
   }
-  return select_paths_v(problem, precision, st, warp_mode, st == 0 && mode2, cv);
+  return select_paths_v(problem, precision, st, warp_mode, alt, cv);
+}
+// FP64 warp mode keeps the function tables (40 KB) in shared memory, but for a
+// CTA of one warp whose patch's nodes leave no room (10,159 nodes and more).
+bool tables_shared(int stencil_kind, int block, size_t slots) {
+  return !(stencil_kind == 2 && block == 32 && sizeof(fx::Tables) + slots > kPathsSmemMax);
 }
 
 }  // namespace
 
 size_t paths_smem_bytes(int precision, int stencil_kind, int acc_words, int smem_nodes, bool warp_mode, int block,
                         bool wm_shared) {
-  if (warp_mode)
-    return (precision == 0 ? sizeof(fx::Tables) : 0) +
-           static_cast<size_t>(block / 32) * paths_slot_bytes(precision, stencil_kind, wm_shared ? acc_words : 0, smem_nodes);
+  if (warp_mode) {
+    const size_t slots = static_cast<size_t>(block / 32) * paths_slot_bytes(precision, stencil_kind, wm_shared ? acc_words : 0, smem_nodes);
+    return slots + (precision == 0 && tables_shared(stencil_kind, block, slots) ? sizeof(fx::Tables) : 0);
+  }
   return static_cast<size_t>(paths_slots(precision)) * paths_slot_bytes(precision, stencil_kind, acc_words, smem_nodes);
 }
 
 cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int grid, int block, size_t smem,
                          cudaStream_t s, bool warp_mode) {
   if (block < 32 || block > 256 || block % 32 != 0) return cudaErrorInvalidValue;
-  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0,
-                                a.mix && (precision == 1 || a.n_cls > 1));
+  bool alt = a.stencil_kind == 0 && a.mix && (precision == 1 || a.n_cls > 1);
+  if (warp_mode && precision == 0 && a.stencil_kind == 2)
+    alt = !tables_shared(2, block, static_cast<size_t>(block / 32) * paths_slot_bytes(0, 2, 0, a.smem_nodes));
+  const void* fn = select_paths(problem, precision, a.stencil_kind, warp_mode, block, smem, a.any_cv != 0, alt);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<LaunchArgs*>(&a)};
@@ -53,7 +61,7 @@ cudaError_t launch_paths(const LaunchArgs& a, int problem, int precision, int gr
 
 int paths_kernel_occupancy(int problem, int precision, int stencil_kind, int cv, int block, size_t smem, bool warp_mode,
                            bool stream) {
-  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0, stream);
+  const void* fn = select_paths(problem, precision, stencil_kind, warp_mode, block, smem, cv != 0, stencil_kind == 0 && stream);
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess) return 1;

@@ -783,8 +783,10 @@ __device__ __forceinline__ void add_arc_moments(double* acc, unsigned im, double
 // warp mode and the larger patches of the 32x32 mesh measured slower at 64
 // registers.
 // MODE (warp mode): 0 the warp drains at the end of every chunk; 1 streaming
-// (below); 2 streaming with several classes of chunks.  FP64 always streams;
-// FP32 only in point solves of many paths per item: its thread sums round to
+// (below); 2 streaming with several classes of chunks; 3 as 2 with the FP64
+// function tables in global memory, where a patch's nodes take their place.
+// FP64 always streams; FP32 only in point solves of many paths per item (and
+// those without allocation, whose paths the host does not know): its thread sums round to
 // 2^-24 of a path's score at every addition, so another partition of the paths
 // moves a mean of a few hundred by 4e-9, and its stencil launches form their
 // rows per item in the kernel.  Mode 1 is for FP64 point solves of one class:
@@ -795,9 +797,9 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
   using SAcc = typename std::conditional<WM, double, typename SAccType<R, ST>::type>::type;
   using Acc = typename std::conditional<std::is_same<R, double>::value, AccD, AccK>::type;
   constexpr int kPrec = std::is_same<R, double>::value ? 0 : 1;
-  constexpr bool kMix = MODE > 0, CLS = MODE == 2;
+  constexpr bool kMix = MODE > 0, CLS = MODE >= 2;
   // FP64 stepping in warp mode: the function tables at the start of the shared memory
-  constexpr bool kShTab = WM && kPrec == 0;
+  constexpr bool kShTab = WM && kPrec == 0 && MODE != 3;
   constexpr size_t kTab = kShTab ? sizeof(fx::Tables) : 0;
   constexpr int S = WM ? kMaxBlockWarps : (kPrec == 0 ? 2 : kSlotsFP32);  // slots, or one per warp
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1574,8 +1576,8 @@ __global__ void __launch_bounds__(256, MB) paths_kernel(const LaunchArgs a) {
 }
 
 // The kernel instantiation of a launch: stencil kind st (0 points, 1 arcs,
-// 2 patches), `alt` the 4-CTA build of FP32 patch slot mode or the mode 2
-// build of point solves; CV: the build with the
+// 2 patches), `alt` the 4-CTA build of FP32 patch slot mode, the mode 2 build
+// of point solves or the mode 3 build of FP64 patches; CV: the build with the
 // control-variate terms (without them xi = 0 and the VR sums are the plain
 // ones).
 template <typename R, int PROB, bool WM, bool CV>
@@ -1586,6 +1588,8 @@ const void* paths_fn(int st, bool alt) {
   switch (st) {
     case 1: return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 1, WM, MB, CV, MODE>);
     case 2:
+      if constexpr (f64 && WM)
+        if (alt) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV, 3>);
       if constexpr (!f64 && !WM)
         if (alt) return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, 4, CV, 0>);
       return reinterpret_cast<const void*>(&paths_kernel<R, PROB, 2, WM, MB, CV, MODE>);
